@@ -70,7 +70,7 @@ def draw(rng):
     if kind == "lattice":
         return {"kind": kind, "side": int(_log(rng, 40, 990)), "mixed": mixed}
     if kind == "serve":
-        return {"kind": kind, "sizes": " ".join(str(int(_log(rng, 5000, 60000))) for _ in range(rng.randint(1, 3))),
+        return {"kind": kind, "sizes": " ".join(str(int(_log(rng, 5000, 30000))) for _ in range(rng.randint(1, 3))),
                 "steps": rng.randint(3, 10)}
     solver = rng.choice(["bicgstab_device", "bicgstab_device", "fgmres_host", "bicgstab_host"])
     return {"kind": kind, "n": int(_log(rng, 60, 65000 if solver == "bicgstab_device" else 20000)), "solver": solver}
