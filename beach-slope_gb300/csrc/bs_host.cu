@@ -72,10 +72,12 @@ struct bs_ctx {
     SceneDyn* h_snapdyn = nullptr;
     // multigrid levels run as one clustered launch per visit (mg_sub option)
     int mgsub_on = 0, mgsub_level = 0, mgsub_cs = 1, sm_count = 0;
-    // the last two levels of a visit in one block per scene (option mg_tail,
-    // default on: bit-identical to the separate launches): the level it
-    // starts at (0: off or no level qualifies)
-    int mgtail_on = 1, mgtail_level = 0;
+    // the lower levels of a visit on chip, a cluster of thread blocks per
+    // scene (option mg_tail, default on: bit-identical to the separate
+    // launches): the level it starts at (0: off or no level qualifies), the
+    // blocks per cluster and the shared memory of a block
+    int mgtail_on = 1, mgtail_level = 0, mgchip_cs = 1, mgchip_smem = 0;
+    size_t chip_img_bytes = 0;   // size of D.mg.chip_img
     // FGMRES basis as double-float (hi, lo) FP32 pairs in the preconditioned mixed solve
     int fg_df_on = 1;
     // option "mg_fp32": the FP64 form's multigrid preconditioner in FP32 (the
@@ -206,6 +208,8 @@ bs::Launch launch_of(bs_ctx* c) {
     L.mgneed = c->mgneed.empty() ? nullptr : c->mgneed.data();
     L.mgsub_level = c->mgsub_level;
     L.mgtail = c->mgtail_level;
+    L.mgchip_cs = c->mgchip_cs;
+    L.mgchip_smem = c->mgchip_smem;
     L.mgsub_cs = c->mgsub_cs;
     L.sweep_tpb = c->sweep_tpb;
     L.mg0_tpb = c->mg0_tpb;
@@ -264,27 +268,61 @@ void mg_sub_choose(bs_ctx* c) {
     }
 }
 
-// The level whose visits run with the coarsest level in one block per scene
-// (k_mg_tail): every scene that has it has its coarsest level right below it,
-// with at most 1024 cells on it and 256 on the coarsest; 0 when none does or
-// the option, the exact coarse solve or the clustered subtree is on.
+// The level whose visits run on chip with everything below it (k_mg_chip), a
+// cluster of thread blocks per scene: the finest one whose scenes' levels all
+// fit the blocks' shared memory (0: the option is off or none does).  The
+// clusters of a batch share the SMs, so that all of them run at once; a block
+// takes about BS_CHIP_CELLS cells of the first level, where a level operation
+// costs about as much as the barrier behind it.
+#define BS_CHIP_CELLS 1024
 int coarsest_level(const bs_ctx* c, int s);
 void mg_tail_choose(bs_ctx* c) {
     const MgDev& M = c->D.mg;
     c->mgtail_level = 0;
+    c->mgchip_cs = 1;
+    c->mgchip_smem = 0;
     if (!c->mgtail_on || M.exact || c->mgsub_level || c->mglev.empty()) return;
-    for (int l = 1; l < M.nlev; ++l) {
-        bool ok = true, any = false;
-        for (int s = 0; s < c->nscene && ok; ++s) {
-            if (coarsest_level(c, s) < l) continue;
-            any = true;
-            const int mf = c->mglev[l].nx[s] * c->mglev[l].ny[s], mc = c->mglev[l + 1].nx[s] * c->mglev[l + 1].ny[s];
-            ok = coarsest_level(c, s) == l + 1 && mf <= 1024 && mc <= 256;
+    const int prec = mg_prec_of(c);
+    for (int l = 1; l <= M.nlev; ++l) {
+        if (!(c->mgneed[l] & 1)) break;
+        if (!bs::mg_chip_ops_fit(c->D, launch_of(c), l, l > 1 && l - 1 <= M.wlev ? 2 : 1)) continue;
+        int best = 0, best_smem = 0;
+        for (int cs = 1; cs <= 16 && (cs == 1 || cs * c->nscene <= c->sm_count); cs *= 2) {
+            size_t smem = 0;
+            int cells = 0;
+            bool ok = true;
+            for (int s = 0; s < c->nscene && ok; ++s) {
+                const int lc = coarsest_level(c, s);
+                if (lc < l) continue;
+                const int nx = c->mglev[l].nx[s], ny = c->mglev[l].ny[s];
+                if (nx == 0) continue;
+                const size_t b = bs::mg_chip_bytes(prec, lc - l + 1, nx, ny, cs);
+                ok = b > 0 && b <= BS_CHIP_SMEM;
+                smem = std::max(smem, b);
+                cells = std::max(cells, nx * ny / cs);
+            }
+            if (!ok || smem == 0 || !bs::mg_chip_prepare(prec, cs, smem)) continue;
+            best = cs;
+            best_smem = (int)smem;
+            if (cells <= BS_CHIP_CELLS) break;
         }
-        if (ok && any) {
-            c->mgtail_level = l;
-            return;
+        if (!best) continue;
+        best_smem = (best_smem + 15) & ~15;
+        const size_t need = (size_t)c->nscene * best * best_smem;
+        if (need > c->chip_img_bytes) {
+            char* img = (char*)c->D.mg.chip_img;
+            cudaStreamSynchronize(c->stream);
+            dfree(c, img);
+            c->D.mg.chip_img = nullptr;
+            c->chip_img_bytes = 0;
+            if (dalloc(c, &img, need)) return;   // no room: the separate launches
+            c->D.mg.chip_img = img;
+            c->chip_img_bytes = need;
         }
+        c->mgtail_level = l;
+        c->mgchip_cs = best;
+        c->mgchip_smem = best_smem;
+        return;
     }
 }
 
@@ -1736,7 +1774,7 @@ std::vector<unsigned char> step_key(const bs_ctx* c, int flags) {
     const int v[] = {flags, c->precision, c->prm[0].ppe_solver, c->prm[0].ppe_restart, c->prm[0].ppe_precond,
                      c->prm[0].mixed_max_outer, max_ppe_maxit(c), c->mgsub_on, c->mgsub_level, c->mgsub_cs,
                      c->fg_df_on, c->disp_ready ? 1 : 0, any_scalar_on(c) ? 1 : 0, c->nblk_total,
-                     c->sweep_tpb, c->mg0_tpb, c->mg_fp32, c->mgtail_level};
+                     c->sweep_tpb, c->mg0_tpb, c->mg_fp32, c->mgtail_level, c->mgchip_cs, c->mgchip_smem};
     key_put(k, v);
     for (const auto& m : c->mglev) key_put(k, m);
     k.insert(k.end(), c->mgneed.begin(), c->mgneed.end());

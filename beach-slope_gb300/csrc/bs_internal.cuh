@@ -108,6 +108,7 @@ struct MgDev {
     // its first level of at most BS_MG_EXACT_MAX cells, whose operator is
     // inverted once per step; the visits apply the inverse
     int exact;
+    void* chip_img;                   // per scene and block of its cluster: the constants of k_mg_chip
     void* ainv;                       // per scene: BS_MG_EXACT_MAX^2 values (the level's precision), row-major
     double* xinv;                     // per scene: BS_MG_EXACT_MAX^2 doubles (the factorisation's work space)
 };
@@ -559,6 +560,16 @@ struct MgSub {
     unsigned char op[BS_MG_MAXOPS], lv[BS_MG_MAXOPS], acc[BS_MG_MAXOPS];   // op: 0 down, 1 resid, 2 up, 3 coarse
     MgLevel G[BS_MG_SUBL];           // levels l0 .. l0 + BS_MG_SUBL - 1
 };
+// A launch of the levels from l0 down on chip (k_mg_chip): the visit's op
+// list (as MgSub) and, per scene, the first level's grid, the coarsest level
+// and the first cell on each level.
+#define BS_CHIP_SMEM (200 * 1024)    // most shared memory a block of it takes
+struct MgChip {
+    int l0, nops, cs, stride;         // stride: bytes of a block's constants in MgDev::chip_img (its shared memory)
+    unsigned char op[BS_MG_MAXOPS], lv[BS_MG_MAXOPS], acc[BS_MG_MAXOPS];
+    int nx[BS_MG_MAXS], ny[BS_MG_MAXS], lev[BS_MG_MAXS], off[BS_MG_SUBL][BS_MG_MAXS];
+    int d[BS_MG_MAXS], zero[BS_MG_MAXS], zero0[BS_MG_MAXS], img[BS_MG_MAXS], img0[BS_MG_MAXS];   // ChipGeo
+};
 struct Launch {
     cudaStream_t stream;
     int nblk_rows;      // total row blocks
@@ -570,7 +581,8 @@ struct Launch {
     const unsigned char* mgneed;   // per level: bit0 some scene visits it, bit1 restriction and
                                    // prolongation to the next level, bit2 coarsest-level solve
     int mgsub_level, mgsub_cs;     // first level of the clustered subtree (0: per-level launches), CTAs per cluster
-    int mgtail;                    // level whose visits run with the coarsest level in one block (0: none)
+    int mgtail;                    // level whose visits run on chip, everything below included (0: none)
+    int mgchip_cs, mgchip_smem;    // ... blocks per cluster and bytes of shared memory per block
     int sweep_tpb;                 // threads per block of the neighbour sweeps (64, 128 or 256)
     int mg0_tpb;                   // threads per block of the particle-level multigrid kernels
     const MgExact* exact;          // the scenes' exactly solved levels (when D.mg.exact)
@@ -680,7 +692,11 @@ void solve_fp64(const Dev& D, const Launch& L, int maxit, int check_every, int p
                 int* d_all_conv, int* h_all_conv_pinned, cudaEvent_t ev);
 // multigrid preconditioner (bs_mg.cu)
 void mg_setup(const Dev& D, const Launch& L, int mg_precision);
-void mg_apply(const Dev& D, const Launch& L, int mg_precision, const double* in, double* out);
+// (fg: inside FGMRES, whose scenes also rest when their restart cycle has ended)
+void mg_apply(const Dev& D, const Launch& L, int mg_precision, const double* in, double* out, int fg);
+size_t mg_chip_bytes(int mg_precision, int nl, int nx, int ny, int cs);
+bool mg_chip_ops_fit(const Dev& D, const Launch& L, int l0, int visits);
+bool mg_chip_prepare(int mg_precision, int cs, size_t smem);
 // the level-0 input of the V-cycle, written by the Krylov streams (x = p or s)
 template <typename T>
 __device__ __forceinline__ void mg_put_input(const Dev& D, int r, double x) {

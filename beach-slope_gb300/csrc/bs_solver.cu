@@ -1207,14 +1207,14 @@ void solve_fp64(const Dev& D, const Launch& L, int maxit, int check_every, int p
         int q2 = tbegin(L, K_BICG_PUPD);
         launch_pdl(L, k_pupd64, L.nblk_rows, BS_THREADS, 0, D, mgmode);
         tend(L, q2);
-        if (precond) mg_apply(D, L, mg_prec, D.sp, D.sp2);
+        if (precond) mg_apply(D, L, mg_prec, D.sp, D.sp2, 0);
         q2 = tbegin(L, K_BICG_IT1);
         launch_pdl(L, k_it1_64, L.nblk_rows, BS_THREADS, 0, D, pu);
         tend(L, q2);
         q2 = tbegin(L, K_BICG_SUPD);
         launch_pdl(L, k_supd64, L.nblk_rows, BS_THREADS, 0, D, mgmode);
         tend(L, q2);
-        if (precond) mg_apply(D, L, mg_prec, D.ss, D.sv2);
+        if (precond) mg_apply(D, L, mg_prec, D.ss, D.sv2, 0);
         q2 = tbegin(L, K_BICG_IT2);
         launch_pdl(L, k_it2_64, L.nblk_rows, BS_THREADS, 0, D, su);
         tend(L, q2);
@@ -1299,7 +1299,7 @@ void solve_fgmres(const Dev& D, const Launch& L, int maxit, int check_every, int
     };
     auto column = [&]() {
         if (!D.fg_df) put();
-        if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.sp2);
+        if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.sp2, 1);
         int q2 = tbegin(L, K_FG_ARN);
         if (D.fg_df) launch_pdl(L, k_fg_arn1<1>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
         else launch_pdl(L, k_fg_arn1<0>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
@@ -1498,14 +1498,14 @@ void bicg_iteration(const Dev& D, const Launch& L, int precond, int mg_prec, int
     int q = tbegin(L, K_BICG_PUPD);
     launch_pdl(L, k_pupd64, L.nblk_rows, BS_THREADS, 0, D, mgmode);
     tend(L, q);
-    if (precond) mg_apply(D, L, mg_prec, D.sp, D.sp2);
+    if (precond) mg_apply(D, L, mg_prec, D.sp, D.sp2, 0);
     q = tbegin(L, K_BICG_IT1);
     launch_pdl(L, k_it1_64, L.nblk_rows, BS_THREADS, 0, D, pu);
     tend(L, q);
     q = tbegin(L, K_BICG_SUPD);
     launch_pdl(L, k_supd64, L.nblk_rows, BS_THREADS, 0, D, mgmode);
     tend(L, q);
-    if (precond) mg_apply(D, L, mg_prec, D.ss, D.sv2);
+    if (precond) mg_apply(D, L, mg_prec, D.ss, D.sv2, 0);
     q = tbegin(L, K_BICG_IT2);
     launch_pdl(L, k_it2_64, L.nblk_rows, BS_THREADS, 0, D, su);
     tend(L, q);
@@ -1522,7 +1522,7 @@ void fg_put(const Dev& D, const Launch& L, int mgmode) {
 
 void fg_column(const Dev& D, const Launch& L, int precond, int mg_prec, int mgmode, int* d_nconv) {
     if (!D.fg_df) fg_put(D, L, mgmode);
-    if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.sp2);
+    if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.sp2, 1);
     int q = tbegin(L, K_FG_ARN);
     if (D.fg_df) launch_pdl(L, k_fg_arn1<1>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
     else launch_pdl(L, k_fg_arn1<0>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);

@@ -341,10 +341,9 @@ int bs_write_combined(struct bs_ctx* ctx, int32_t scene, const char* fluid_path,
  * default 0: the FP64 form's multigrid preconditioner in FP32 like the mixed
  * form's; the Krylov solve, its residuals and stopping test stay FP64, so the
  * pressure solves the same FP64 system to the same tolerance), "mg_tail" (0/1,
- * default 1: each visit of the level above the coarsest, with the coarsest
- * solve, as one block per scene in shared memory -- bit-identical to the
- * separate launches; used where every scene ends on the same two levels of at
- * most 1024 and 256 cells), "sweep_tpb" /
+ * default 1: the levels of a visit from "mg_tail_level" down as one launch, a
+ * thread-block cluster per scene with every level in its shared memory --
+ * bit-identical to the separate launches), "sweep_tpb" /
  * "mg0_tpb" (64, 128 or 256 threads per block of the neighbour sweeps / of
  * the particle-level multigrid kernels; every row is computed the same way
  * whatever the block size), "step_graph" (0/1, default 1: each bs_step is
