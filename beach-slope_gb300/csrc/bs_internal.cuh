@@ -73,6 +73,10 @@ struct SceneDyn {                 // per-scene dynamic state (device)
     int fg_j, fg_state, fg_k;
     int asm_split;                 // 1: the mixed assembly wrote aval32/aval_lo with aval (k_mx_convert skips the split)
     double fg_rinv;                // 1 / the norm of the vector the next column normalises
+    // double-float basis: the column pass 1 finished (pass 2 projects it and runs its rotations), whether
+    // there is one, whether its norm was not trusted, and that norm
+    int fg_c, fg_act, fg_bad, fg_pad;
+    double fg_hn;
 };
 
 // Aggregation multigrid over the cell grid.  Level 1 = half-cells (2h x 2h,

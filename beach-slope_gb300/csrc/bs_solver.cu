@@ -614,24 +614,34 @@ __device__ __forceinline__ float2 df_shfl_xor(float2 a, int m) {
 
 // Sum `cnt` rows of nv partials (row stride ld) in a fixed order: thread t
 // takes value t % nv over rows q, q+Q, ... (q = t / nv, Q = 256 / nv), the
-// Q sub-sums are added in q order.  Rows of zeros at the end change nothing,
-// so a scene's sums do not depend on its slot's capacity.
-__device__ __forceinline__ void fg_sum_rows(const double* __restrict__ src, int cnt, int ld, int nv, double* out,
+// Q sub-sums are added in q order.  The rows from `have` on are zeros (blocks
+// without rows write nothing): they change nothing, so a scene's sums do not
+// depend on its slot's capacity.  Eight loads in flight per thread.
+__device__ __forceinline__ void fg_sum_rows(const double* __restrict__ src, int cnt, int have, int ld, int nv, double* out,
                                             double* scratch /*[BS_THREADS]*/) {
     const int t = threadIdx.x;
     if (nv <= BS_THREADS) {
         const int Q = BS_THREADS / nv;
         const int i = t % nv, q = t / nv;
         if (q < Q) {
+            // four sub-sums over the rows that come in fours, the rest into the first; no operation for a row
+            // of zeros (an FP64 instruction of a warp takes the SM's FP64 pipe 16 cycles)
+            const int m = cnt > q ? (cnt - q + Q - 1) / Q : 0, full = m & ~3;
+            const int mh = have > q ? (have - q + Q - 1) / Q : 0;
             double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-            int b = q;
-            for (; b + 3 * Q < cnt; b += 4 * Q) {   // four loads in flight per thread
-                a0 += __ldcg(src + (long)b * ld + i);
-                a1 += __ldcg(src + (long)(b + Q) * ld + i);
-                a2 += __ldcg(src + (long)(b + 2 * Q) * ld + i);
-                a3 += __ldcg(src + (long)(b + 3 * Q) * ld + i);
+            for (int k = 0; k < mh; k += 8) {
+                double v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = k + u < mh ? __ldcg(src + (long)(q + (k + u) * Q) * ld + i) : 0.0;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (k + u >= mh) break;
+                    if ((u & 3) == 0 || k + u >= full) a0 += v[u];
+                    else if ((u & 3) == 1) a1 += v[u];
+                    else if ((u & 3) == 2) a2 += v[u];
+                    else a3 += v[u];
+                }
             }
-            for (; b < cnt; b += Q) a0 += __ldcg(src + (long)b * ld + i);
             scratch[q * nv + i] = (a0 + a1) + (a2 + a3);
         }
         __syncthreads();
@@ -642,51 +652,68 @@ __device__ __forceinline__ void fg_sum_rows(const double* __restrict__ src, int 
         }
     } else {
         for (int i = t; i < nv; i += BS_THREADS) {
+            const int full = cnt & ~1;
             double a0 = 0.0, a1 = 0.0;
-            int b = 0;
-            for (; b + 1 < cnt; b += 2) {
-                a0 += __ldcg(src + (long)b * ld + i);
-                a1 += __ldcg(src + (long)(b + 1) * ld + i);
+            for (int k = 0; k < have; k += 8) {
+                double v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = k + u < have ? __ldcg(src + (long)(k + u) * ld + i) : 0.0;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (k + u >= have) break;
+                    if ((u & 1) && k + u < full) a1 += v[u];
+                    else a0 += v[u];
+                }
             }
-            if (b < cnt) a0 += __ldcg(src + (long)b * ld + i);
             out[i] = a0 + a1;
         }
     }
     __syncthreads();
 }
 
-// Two-level scene sum of nv per-block values in vals[] (shared): the last
-// block of each group of 32 row blocks sums the group, the last group of the
-// scene sums the groups into tot[] (shared); true in that block.
-__device__ __forceinline__ bool fg_scene_sum(const Dev& D, int s, int nv, const double* vals, double* tot) {
-    __shared__ double scratch[BS_THREADS];
+// The block's writes reach the device before its count: the writes are ordered
+// before thread 0 by the block barrier and before the count by its fence; true
+// in the block that counts last (its reads come after the others' writes).
+__device__ __forceinline__ bool fg_count(int* counter, int total) {
     __shared__ int last;
-    const ScenePar& P = D.par[s];
-    const int ld = bs::fg_part_ld(D.fg_m);
-    const int lb = blockIdx.x - P.blk0, grp = lb >> 5;
-    const int gsize = min(32, P.nblk - (grp << 5));
-    double* part = D.fg_part + (long)blockIdx.x * ld;
-    for (int i = threadIdx.x; i < nv; i += BS_THREADS) part[i] = vals[i];
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(&D.fg_gdone[P.grp0 + grp], 1) == gsize - 1);
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    fg_sum_rows(D.fg_part + (long)(P.blk0 + (grp << 5)) * ld, gsize, ld, nv, tot, scratch);
-    double* gp = D.fg_gpart + (long)(P.grp0 + grp) * ld;
-    for (int i = threadIdx.x; i < nv; i += BS_THREADS) gp[i] = tot[i];
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        D.fg_gdone[P.grp0 + grp] = 0;
-        last = (atomicAdd(&D.blk_done[s], 1) == ((P.nblk + 31) >> 5) - 1);
+        __threadfence();
+        last = atomicAdd(counter, 1) == total - 1;
+        if (last) {
+            *counter = 0;
+            __threadfence();
+        }
     }
     __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    fg_sum_rows(D.fg_gpart + (long)P.grp0 * ld, (P.nblk + 31) >> 5, ld, nv, tot, scratch);
-    if (threadIdx.x == 0) D.blk_done[s] = 0;
+    return last != 0;
+}
+
+// Two-level scene sum of nv per-block values in vals[] (shared) over the
+// scene's nact blocks that hold rows: the last block of each group of 32 row
+// blocks sums the group, the last group of the scene sums the groups into
+// tot[] (shared); true in that block.  one_level: a small scene's last block
+// sums them all (the order of the sums differs, so only where the solve does
+// not multiply such a difference: without the FP32 preconditioner).
+#define BS_FG_ONE_LEVEL 64
+__device__ __forceinline__ bool fg_scene_sum(const Dev& D, int s, int nact, int nv, const double* vals, double* tot,
+                                             bool one_level) {
+    __shared__ double scratch[BS_THREADS];
+    const ScenePar& P = D.par[s];
+    const int ld = bs::fg_part_ld(D.fg_m);
+    const int grp = (blockIdx.x - P.blk0) >> 5, ngrp = (nact + 31) >> 5;
+    double* part = D.fg_part + (long)blockIdx.x * ld;
+    for (int i = threadIdx.x; i < nv; i += BS_THREADS) part[i] = vals[i];
+    one_level = one_level && nact <= BS_FG_ONE_LEVEL;
+    const int have = one_level ? nact : min(32, nact - (grp << 5));
+    if (!fg_count(one_level ? &D.blk_done[s] : &D.fg_gdone[P.grp0 + grp], have)) return false;
+    const double* src = D.fg_part + (long)(P.blk0 + (one_level ? 0 : grp << 5)) * ld;
+    fg_sum_rows(src, one_level ? nact : min(32, P.nblk - (grp << 5)), have, ld, nv, tot, scratch);
+    if (one_level) return true;
+    double* gp = D.fg_gpart + (long)(P.grp0 + grp) * ld;
+    for (int i = threadIdx.x; i < nv; i += BS_THREADS) gp[i] = tot[i];
+    if (!fg_count(&D.blk_done[s], ngrp)) return false;
+    fg_sum_rows(D.fg_gpart + (long)P.grp0 * ld, (P.nblk + 31) >> 5, ngrp, ld, nv, tot, scratch);
     return true;
 }
 
@@ -759,46 +786,99 @@ __global__ void k_fg_put(Dev D, int mgmode) {
     else if (mgmode == 2) bs::mg_put_input<float>(D, r, v);
 }
 
-// Column finisher (one block, the scene's last): the new column h[0..j] of
-// H, with h_{j+1,j} = hn below it, rotated by the cycle's earlier Givens
-// rotations (staged in shared memory; the sweep, a dependent chain, run by
-// one thread), a new rotation that zeroes hn, the residual estimate
-// |g_{j+1}| and the cycle's state.  est: hn was formed from the Gram
+// Column finisher (one block per scene): the new column h[0..j] of H, with
+// h_{j+1,j} = hn below it, rotated by the cycle's earlier Givens rotations, a
+// new rotation that zeroes hn, the residual estimate |g_{j+1}| and the cycle's
+// state.  The value that runs down the column obeys t_{i+1} = -sn_i t_i +
+// cs_i h_{i+1}.  scan: this chain of affine maps is composed by a prefix scan
+// over the lanes of one warp (one after another they take 10 us at column 150);
+// else one thread runs down it (in a block beside pass 2's streaming blocks,
+// where its time does not count).  est_bad: hn was formed from the Gram
 // relation rather than summed, and was not trusted (cancellation), so the
 // cycle restarts from the true residual instead of going on.
-__device__ void fg_finish_column(const Dev& D, int s, const FgSmall& f, int j, double hn, bool est_bad, int* nconv) {
-    __shared__ double hcol[BS_FG_MAXM + 2], csh[BS_FG_MAXM], snh[BS_FG_MAXM];
+__device__ void fg_finish_column(const Dev& D, int s, const FgSmall& f, int j, double hn, bool est_bad, bool scan,
+                                 int* nconv) {
+    constexpr int PER = (BS_FG_MAXM + 31) / 32;   // rotations per lane
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
     const ScenePar& P = D.par[s];
     const int m = D.fg_m;
     double* h = f.H + (long)j * (m + 1);
-    for (int i = threadIdx.x; i <= j; i += BS_THREADS) hcol[i] = h[i];
-    for (int i = threadIdx.x; i < j; i += BS_THREADS) {
-        csh[i] = f.cs[i];
-        snh[i] = f.sn[i];
+    double c[PER], sn[PER], b[PER];
+    const int per = (j + 31) / 32, i0 = lane * per;   // this lane's rotations [i0, i0 + per) below j
+    const double first = __ldcg(h);
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const bool in = q < per && i0 + q < j;
+        c[q] = in ? __ldcg(f.cs + i0 + q) : 1.0;
+        sn[q] = in ? __ldcg(f.sn + i0 + q) : 0.0;
+        b[q] = in ? __ldcg(h + i0 + q + 1) : 0.0;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        SceneDyn& Y = D.dyn[s];
-        double hi = hcol[0];
-        for (int i = 0; i < j; ++i) {   // earlier rotations on the new column
-            const double b = hcol[i + 1];
-            hcol[i] = csh[i] * hi + snh[i] * b;
-            hi = -snh[i] * hi + csh[i] * b;
+    const double gj = lane == 0 ? __ldcg(f.g + j) : 0.0;
+    double a;
+    if (scan) {
+        // the lane's map t -> A t + C over its rotations; a rotation beyond j leaves t as it is
+        double A = 1.0, C = 0.0;
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            if (q >= per || i0 + q >= j) continue;
+            A = -sn[q] * A;
+            C = -sn[q] * C + c[q] * b[q];
         }
-        const double a = hi;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {   // inclusive scan: the maps of lanes 0 .. lane
+            const double Ap = __shfl_up_sync(0xffffffffu, A, o), Cp = __shfl_up_sync(0xffffffffu, C, o);
+            if (lane >= o) {
+                C = A * Cp + C;
+                A = A * Ap;
+            }
+        }
+        const double end = A * first + C;   // after this lane's rotations
+        double t = __shfl_up_sync(0xffffffffu, end, 1);
+        if (lane == 0) t = first;
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            if (q >= per || i0 + q >= j) continue;
+            h[i0 + q] = c[q] * t + sn[q] * b[q];
+            t = -sn[q] * t + c[q] * b[q];
+        }
+        a = __shfl_sync(0xffffffffu, end, 31);
+    } else {
+        __shared__ double hcol[BS_FG_MAXM + 1], csh[BS_FG_MAXM], snh[BS_FG_MAXM];
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+            if (q < per && i0 + q < j) {
+                csh[i0 + q] = c[q];
+                snh[i0 + q] = sn[q];
+                hcol[i0 + q + 1] = b[q];
+            }
+        __syncwarp();
+        a = first;
+        if (lane == 0) {
+            double hi = first;
+            for (int i = 0; i < j; ++i) {
+                const double bi = hcol[i + 1];
+                hcol[i] = csh[i] * hi + snh[i] * bi;
+                hi = -snh[i] * hi + csh[i] * bi;
+            }
+            a = hi;
+        }
+        __syncwarp();
+        for (int i = lane; i < j; i += 32) h[i] = hcol[i];
+    }
+    if (lane == 0) {
+        SceneDyn& Y = D.dyn[s];
         const double den = sqrt(a * a + hn * hn);
-        const double c = den > 0.0 ? a / den : 1.0, sn = den > 0.0 ? hn / den : 0.0;
-        f.cs[j] = c;
-        f.sn[j] = sn;
-        hcol[j] = den;
-        hcol[j + 1] = 0.0;
-        const double gj = f.g[j];
-        f.g[j] = c * gj;
-        f.g[j + 1] = -sn * gj;
-        const double res = fabs(f.g[j + 1]);
+        const double cc = den > 0.0 ? a / den : 1.0, ss = den > 0.0 ? hn / den : 0.0;
+        f.cs[j] = cc;
+        f.sn[j] = ss;
+        h[j] = den;
+        h[j + 1] = 0.0;
+        f.g[j] = cc * gj;
+        f.g[j + 1] = -ss * gj;
+        const double res = fabs(ss * gj);
         Y.rnorm2 = res * res;
         Y.rho_old = hn;
-        Y.fg_rinv = hn > 0.0 ? 1.0 / hn : 0.0;
         Y.iters += 1;
         Y.fg_j = j + 1;
         int st = 0;
@@ -817,8 +897,6 @@ __device__ void fg_finish_column(const Dev& D, int s, const FgSmall& f, int j, d
         Y.fg_state = st;
         if (st) atomicAdd(nconv, 1);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i <= j + 1; i += BS_THREADS) h[i] = hcol[i];
 }
 
 // s += (a.x + a.y) z for an FP32 z: TwoProduct of the high part, the low
@@ -930,7 +1008,12 @@ template <int DF>
 __global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond, int* nconv) {
     BS_PDL_ENTRY();
     const int s = D.blk_scene[blockIdx.x];
-    if (!fg_running(D, s)) return;
+    if (!fg_running(D, s)) {
+        if (DF && (int)blockIdx.x == D.par[s].blk0 && threadIdx.x == 0) D.dyn[s].fg_act = 0;   // no column for pass 2
+        return;
+    }
+    const int nact = (D.dyn[s].n + BS_THREADS - 1) / BS_THREADS;
+    if ((int)blockIdx.x - D.par[s].blk0 >= nact) return;   // no rows
     __shared__ double ws[BS_THREADS], vs[BS_THREADS];
     __shared__ double dsh[2 * (BS_FG_MAXM + 1)];
     __shared__ double tsh[2 * (BS_FG_MAXM + 1)];
@@ -1007,57 +1090,86 @@ __global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond, i
     }
     }
     __syncthreads();
-    if (!fg_scene_sum(D, s, DF ? 2 * nv + 1 : 2 * nv, dsh, tsh)) return;
+    if (!fg_scene_sum(D, s, nact, DF ? 2 * nv + 1 : 2 * nv, dsh, tsh, !precond)) return;
     const FgSmall f = fg_small(D, s);
     const int ldg = D.fg_m + 1;
     for (int i = threadIdx.x; i < nv; i += BS_THREADS) {
         f.Gm[i + (long)j * ldg] = tsh[nv + i];
         f.Gm[j + (long)i * ldg] = tsh[nv + i];
     }
-    __syncthreads();
-    // hc = (2I - Gm) h, a warp per row: Gm is symmetric, so row i is read as
-    // the contiguous column i (coalesced, a few loads per lane)
-    __shared__ double hcs[BS_FG_MAXM + 1];
+    // Gm x for a vector x in shared memory, rows wid, wid + 8, ... by warp, four
+    // rows' loads in flight (Gm is symmetric: row i is read as the contiguous
+    // column i; its new row and column from tsh), the four sums over the lanes by
+    // one transposing butterfly (6 FP64 adds instead of 20: this block's FP64
+    // pipe sets its time); put(i, value) in one lane
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int i = wid; i < nv; i += BS_THREADS / 32) {
-        const double* gcol = f.Gm + (long)i * ldg;
-        double a = 0.0;
-        for (int k = lane; k < nv; k += 32) a += __ldcg(gcol + k) * tsh[k];
-        a = warp_sum(a);
-        if (lane == 0) {
-            const double acc = 2.0 * tsh[i] - a;
-            f.hc[i] = acc;
-            f.H[i + (long)j * ldg] = acc;
-            hcs[i] = acc;
+    auto gram = [&](const double* x, auto&& put) {
+        for (int i0 = wid; i0 < nv; i0 += 4 * (BS_THREADS / 32)) {
+            double a[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int k = lane; k < nv; k += 32) {
+                double g[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int i = i0 + u * (BS_THREADS / 32);
+                    g[u] = i >= nv ? 0.0 : i == j ? tsh[nv + k] : k == j ? tsh[nv + i] : __ldcg(f.Gm + (long)i * ldg + k);
+                }
+                const double xk = x[k];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (i0 + u * (BS_THREADS / 32) < nv) a[u] += g[u] * xk;
+            }
+            const bool b4 = lane & 16, b3 = lane & 8;
+            double y[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                y[u] = (b4 ? a[u + 2] : a[u]) + __shfl_xor_sync(0xffffffffu, b4 ? a[u] : a[u + 2], 16);
+            double v = (b3 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b3 ? y[0] : y[1], 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 4);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            const int i = i0 + ((b4 ? 2 : 0) + (b3 ? 1 : 0)) * (BS_THREADS / 32);
+            if ((lane & 7) == 0 && i < nv) put(i, v);
         }
-    }
+    };
+    // hc = (2I - Gm) h
+    __shared__ double hcs[BS_FG_MAXM + 1];
+    gram(tsh, [&](int i, double a) {
+        const double acc = 2.0 * tsh[i] - a;
+        f.hc[i] = acc;
+        f.H[i + (long)j * ldg] = acc;
+        hcs[i] = acc;
+    });
     if (!DF) return;
     // h_{j+1,j} = ||w|| for w = u - V c without a pass over w: ||w||^2 =
     // u.u - 2 c.h + c^T Gm c (u = A z_j, h = V^T u, Gm = V^T V, c = hc), so
     // pass 2 can write v_{j+1} and the V-cycle input directly.  When that
     // difference falls below 1e-6 u.u the estimate is not trusted and the
-    // cycle restarts from the true residual.
+    // cycle restarts from the true residual.  Pass 2 also runs the column's
+    // rotations (in a block of its own, beside the streaming ones).
     __shared__ double eparts[BS_THREADS / 32];
-    __shared__ double eta2s;
     __syncthreads();
-    double part = 0.0;
-    for (int i = wid; i < nv; i += BS_THREADS / 32) {
-        const double* gcol = f.Gm + (long)i * ldg;
-        double g = 0.0;
-        for (int k = lane; k < nv; k += 32) g += __ldcg(gcol + k) * hcs[k];
-        g = warp_sum(g);
-        part += hcs[i] * (g - 2.0 * tsh[i]);
+    // (a warp's rows in order, then the warps)
+    __shared__ double gts[BS_FG_MAXM + 1];
+    gram(hcs, [&](int i, double g) { gts[i] = g; });
+    __syncwarp();
+    if (lane == 0) {
+        double part = 0.0;
+        for (int i = wid; i < nv; i += BS_THREADS / 32) part += hcs[i] * (gts[i] - 2.0 * tsh[i]);
+        eparts[wid] = part;
     }
-    if (lane == 0) eparts[wid] = part;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double e = tsh[2 * nv];
-        for (int w = 0; w < BS_THREADS / 32; ++w) e += eparts[w];
-        eta2s = e;
+        const double uu = tsh[2 * nv];
+        double eta2 = uu;
+        for (int w = 0; w < BS_THREADS / 32; ++w) eta2 += eparts[w];
+        const double hn = sqrt(fmax(eta2, 0.0));
+        SceneDyn& Y = D.dyn[s];
+        Y.fg_c = j;
+        Y.fg_hn = hn;
+        Y.fg_bad = !(eta2 > 1e-6 * uu);
+        Y.fg_rinv = hn > 0.0 ? 1.0 / hn : 0.0;
+        Y.fg_act = 1;
     }
-    __syncthreads();
-    const double uu = tsh[2 * nv], eta2 = eta2s;
-    fg_finish_column(D, s, f, j, sqrt(fmax(eta2, 0.0)), !(eta2 > 1e-6 * uu), nconv);
 }
 
 // Column j, pass 2: w -= V hc (the pending vector, into ss), h_{j+1,j} = ||w||;
@@ -1065,17 +1177,26 @@ __global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond, i
 // With the double-float basis (DF): column j = fg_j - 1 was finished by pass
 // 1, and this pass writes v_{j+1} = (w - V hc) / h_{j+1,j} into the basis
 // and the V-cycle input (mgmode as k_fg_put), with no reduction.
+// Its first D.nscene blocks (DF) run the scenes' rotations (fg_finish_column),
+// beside the streaming blocks; these read only what pass 1 left (fg_c, fg_act,
+// fg_rinv), so a cycle that ends with this column has one vector too many.
 template <int DF>
 __global__ void k_fg_arn2(Dev D, int* nconv, int mgmode) {
     BS_PDL_ENTRY();
-    const int s = D.blk_scene[blockIdx.x];
-    if (!fg_running(D, s)) return;
+    if (DF && (int)blockIdx.x < D.nscene) {
+        const SceneDyn& Y = D.dyn[blockIdx.x];
+        if (Y.fg_act) fg_finish_column(D, blockIdx.x, fg_small(D, blockIdx.x), Y.fg_c, Y.fg_hn, Y.fg_bad != 0, false, nconv);
+        return;
+    }
+    const int blk = DF ? blockIdx.x - D.nscene : blockIdx.x;
+    const int s = D.blk_scene[blk];
+    if (DF ? !D.dyn[s].fg_act : !fg_running(D, s)) return;
     __shared__ double hs[BS_FG_MAXM + 1];
     __shared__ float2 hsd[BS_FG_MAXM + 1];
     const ScenePar& P = D.par[s];
-    const int j = DF ? D.dyn[s].fg_j - 1 : D.dyn[s].fg_j;
+    const int j = DF ? D.dyn[s].fg_c : D.dyn[s].fg_j;
     const int rend = P.row0 + D.dyn[s].n;
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = blk * blockDim.x + threadIdx.x;
     const FgSmall f = fg_small(D, s);
     for (int i = threadIdx.x; i <= j; i += BS_THREADS) {
         hs[i] = f.hc[i];
@@ -1121,8 +1242,14 @@ __global__ void k_fg_arn2(Dev D, int* nconv, int mgmode) {
         q[0] = w * w;
     }
     double tot[1];
+    __shared__ double hns;
     if (!scene_sum<1>(D, s, q, tot)) return;
-    fg_finish_column(D, s, f, j, sqrt(tot[0]), false, nconv);
+    if (threadIdx.x == 0) {
+        hns = sqrt(tot[0]);
+        D.dyn[s].fg_rinv = hns > 0.0 ? 1.0 / hns : 0.0;
+    }
+    __syncthreads();
+    fg_finish_column(D, s, f, j, hns, false, mgmode == 0, nconv);   // (a preconditioned solve keeps the plain chain)
 }
 
 // One warp per scene: y = R^-1 g over the cycle's k columns; scenes that
@@ -1305,7 +1432,7 @@ void solve_fgmres(const Dev& D, const Launch& L, int maxit, int check_every, int
         else launch_pdl(L, k_fg_arn1<0>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
         tend(L, q2);
         q2 = tbegin(L, K_FG_ORTH);
-        if (D.fg_df) launch_pdl(L, k_fg_arn2<1>, L.nblk_rows, BS_THREADS, 0, D, d_nconv, mgmode);
+        if (D.fg_df) launch_pdl(L, k_fg_arn2<1>, L.nblk_rows + D.nscene, BS_THREADS, 0, D, d_nconv, mgmode);
         else launch_pdl(L, k_fg_arn2<0>, L.nblk_rows, BS_THREADS, 0, D, d_nconv, mgmode);
         tend(L, q2);
     };
@@ -1528,7 +1655,7 @@ void fg_column(const Dev& D, const Launch& L, int precond, int mg_prec, int mgmo
     else launch_pdl(L, k_fg_arn1<0>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
     tend(L, q);
     q = tbegin(L, K_FG_ORTH);
-    if (D.fg_df) launch_pdl(L, k_fg_arn2<1>, L.nblk_rows, BS_THREADS, 0, D, d_nconv, mgmode);
+    if (D.fg_df) launch_pdl(L, k_fg_arn2<1>, L.nblk_rows + D.nscene, BS_THREADS, 0, D, d_nconv, mgmode);
     else launch_pdl(L, k_fg_arn2<0>, L.nblk_rows, BS_THREADS, 0, D, d_nconv, mgmode);
     tend(L, q);
 }
