@@ -477,6 +477,25 @@ __device__ __forceinline__ CorrF corr_f(const Dev& D, int r) {
     return CorrF{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 }
 
+// ---- thread-block clusters
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// store into the shared memory of the cluster's block `rank`, at the same offset
+__device__ __forceinline__ void st_rank(unsigned p, int rank, float v) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(p), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_rank(unsigned p, int rank, double v) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(p), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
 __device__ __forceinline__ void set_err(const Dev& D, int s, unsigned bits) {
     atomicOr(&D.dyn[s].err, bits);
     atomicOr(D.err_word, bits);

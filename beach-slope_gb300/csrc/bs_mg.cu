@@ -694,13 +694,6 @@ __global__ void __launch_bounds__(BS_CHIP_THREADS) k_mg_chip_pack(Dev D, __grid_
     }
 }
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 // Shared memory by 32-bit address (these chains of short dependent operations
 // are bound by their instruction count).  The order of the accesses of a thread
 // is that of the source.
@@ -736,17 +729,6 @@ __device__ __forceinline__ unsigned sld_u(unsigned a) {
 }
 __device__ __forceinline__ void sst(unsigned a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
 __device__ __forceinline__ void sst(unsigned a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
-// store into the shared memory of the cluster's block `rank`, at the same offset
-__device__ __forceinline__ void st_rank(unsigned p, int rank, float v) {
-    unsigned a;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(p), "r"(rank));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-__device__ __forceinline__ void st_rank(unsigned p, int rank, double v) {
-    unsigned a;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(p), "r"(rank));
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
 // the 4x4 window at p (an even value: two-value loads), W[column][row]
 template <typename T>
 __device__ __forceinline__ void chip_window(unsigned p, int sy, T (&W)[4][4]) {
@@ -1373,8 +1355,8 @@ __global__ void k_mg_l0_up(Dev D, double* __restrict__ out, int mode, int fg) {
     if (mode == 1) {
         ((T*)D.mg.u)[r] = v;
     } else {
-        out[r] = (double)v;
-        if (sizeof(T) == 4 && D.zf) D.zf[r] = (float)v;   // the FGMRES pass reads it in FP32
+        if (out) out[r] = (double)v;
+        if (sizeof(T) == 4 && D.zf) D.zf[r] = (float)v;   // the double-float FGMRES pass reads it in FP32 (out null)
     }
 }
 

@@ -531,11 +531,11 @@ __global__ void k_true_res64(Dev D) {
 // columns serves every cycle.
 //
 // Two forms of a column.  FP64 basis (fg_df = 0): k_fg_put writes v_j and the
-// V-cycle input, pass 1 (k_fg_arn1<0>) the SpMV and the dots, pass 2
+// V-cycle input, pass 1 (k_fg_arn1) the SpMV and the dots, pass 2
 // (k_fg_arn2<0>) the projection, the norm and, in its finisher, the
 // rotations.  Double-float basis (fg_df = 1, the preconditioned mixed solve):
 // the basis is stored as (hi, lo) FP32 pairs and its dots and projection run
-// on the FP32 pipe; pass 1 (k_fg_arn1<1>) also sums u.u and its finisher takes
+// on the FP32 pipe; pass 1 (k_fg_arn1_df) also sums u.u and its finisher takes
 // h_{j+1,j} from the Gram relation and runs the rotations, so pass 2
 // (k_fg_arn2<1>) streams v_{j+1} and the next V-cycle input with no reduction
 // and k_fg_put runs once per cycle.
@@ -690,28 +690,41 @@ __device__ __forceinline__ bool fg_count(int* counter, int total) {
 }
 
 // Two-level scene sum of nv per-block values in vals[] (shared) over the
-// scene's nact blocks that hold rows: the last block of each group of 32 row
-// blocks sums the group, the last group of the scene sums the groups into
-// tot[] (shared); true in that block.  one_level: a small scene's last block
-// sums them all (the order of the sums differs, so only where the solve does
-// not multiply such a difference: without the FP32 preconditioner).
+// scene's nact blocks that hold rows.  First level: the last block of each
+// group of 32 row blocks sums the group into fg_gpart (tot: shared); true in
+// that block.
+__device__ __forceinline__ bool fg_group_sum(const Dev& D, int s, int nact, int nv, const double* vals, double* tot,
+                                             double* scratch /*[BS_THREADS]*/) {
+    const ScenePar& P = D.par[s];
+    const int ld = bs::fg_part_ld(D.fg_m);
+    const int grp = (blockIdx.x - P.blk0) >> 5, have = min(32, nact - (grp << 5));
+    double* part = D.fg_part + (long)blockIdx.x * ld;
+    for (int i = threadIdx.x; i < nv; i += BS_THREADS) part[i] = vals[i];
+    if (!fg_count(&D.fg_gdone[P.grp0 + grp], have)) return false;
+    fg_sum_rows(D.fg_part + (long)(P.blk0 + (grp << 5)) * ld, min(32, P.nblk - (grp << 5)), have, ld, nv, tot, scratch);
+    double* gp = D.fg_gpart + (long)(P.grp0 + grp) * ld;
+    for (int i = threadIdx.x; i < nv; i += BS_THREADS) gp[i] = tot[i];
+    return true;
+}
+// Both levels: the last group of the scene sums the groups into tot[]; true in
+// that block.  one_level: a small scene's last block sums its blocks' values
+// itself (the order of the sums differs, so only where the solve does not
+// multiply such a difference: without the FP32 preconditioner).
 #define BS_FG_ONE_LEVEL 64
 __device__ __forceinline__ bool fg_scene_sum(const Dev& D, int s, int nact, int nv, const double* vals, double* tot,
                                              bool one_level) {
     __shared__ double scratch[BS_THREADS];
     const ScenePar& P = D.par[s];
     const int ld = bs::fg_part_ld(D.fg_m);
-    const int grp = (blockIdx.x - P.blk0) >> 5, ngrp = (nact + 31) >> 5;
-    double* part = D.fg_part + (long)blockIdx.x * ld;
-    for (int i = threadIdx.x; i < nv; i += BS_THREADS) part[i] = vals[i];
-    one_level = one_level && nact <= BS_FG_ONE_LEVEL;
-    const int have = one_level ? nact : min(32, nact - (grp << 5));
-    if (!fg_count(one_level ? &D.blk_done[s] : &D.fg_gdone[P.grp0 + grp], have)) return false;
-    const double* src = D.fg_part + (long)(P.blk0 + (one_level ? 0 : grp << 5)) * ld;
-    fg_sum_rows(src, one_level ? nact : min(32, P.nblk - (grp << 5)), have, ld, nv, tot, scratch);
-    if (one_level) return true;
-    double* gp = D.fg_gpart + (long)(P.grp0 + grp) * ld;
-    for (int i = threadIdx.x; i < nv; i += BS_THREADS) gp[i] = tot[i];
+    if (one_level && nact <= BS_FG_ONE_LEVEL) {
+        double* part = D.fg_part + (long)blockIdx.x * ld;
+        for (int i = threadIdx.x; i < nv; i += BS_THREADS) part[i] = vals[i];
+        if (!fg_count(&D.blk_done[s], nact)) return false;
+        fg_sum_rows(D.fg_part + (long)P.blk0 * ld, nact, nact, ld, nv, tot, scratch);
+        return true;
+    }
+    const int ngrp = (nact + 31) >> 5;
+    if (!fg_group_sum(D, s, nact, nv, vals, tot, scratch)) return false;
     if (!fg_count(&D.blk_done[s], ngrp)) return false;
     fg_sum_rows(D.fg_gpart + (long)P.grp0 * ld, (P.nblk + 31) >> 5, ngrp, ld, nv, tot, scratch);
     return true;
@@ -914,104 +927,109 @@ __device__ __forceinline__ void df_fma1(float2& s, float2 a, float z) {
 
 // Row r of A z for an FP32-exact z (the mixed V-cycle output, zf): the
 // off-diagonal values as double-float pairs (aval32 + aval_lo, 48 bits) and
-// the products and sums on the FP32 pipe; the diagonal term in FP64.
-__device__ __forceinline__ double spmv_row_df(const Dev& D, const float* __restrict__ z, int r) {
+// the products and sums on the FP32 pipe, eight gathers in flight; the diagonal
+// term in FP64.  zr: z of the row in FP64.
+__device__ __forceinline__ double spmv_row_df(const Dev& D, const float* z, int r, double& zr) {
     const float* __restrict__ Ah = D.aval32;
     const float* __restrict__ Al = D.aval_lo;
     const int* __restrict__ idx = D.nidx;
     const int n = D.ncount[r];
+    const float zrow = z[r];
     float2 acc = make_float2(0.f, 0.f);
     long e = ell(r, 0, D.kmax);
     int k = 0;
-    for (; k + 4 <= n; k += 4, e += 128) {   // four independent gathers in flight
-        const int j0 = __ldg(idx + e), j1 = __ldg(idx + e + 32), j2 = __ldg(idx + e + 64), j3 = __ldg(idx + e + 96);
-        const float2 a0 = make_float2(__ldg(Ah + e), __ldg(Al + e));
-        const float2 a1 = make_float2(__ldg(Ah + e + 32), __ldg(Al + e + 32));
-        const float2 a2 = make_float2(__ldg(Ah + e + 64), __ldg(Al + e + 64));
-        const float2 a3 = make_float2(__ldg(Ah + e + 96), __ldg(Al + e + 96));
-        const float z0 = z[j0], z1 = z[j1], z2 = z[j2], z3 = z[j3];
-        df_fma1(acc, a0, z0);
-        df_fma1(acc, a1, z1);
-        df_fma1(acc, a2, z2);
-        df_fma1(acc, a3, z3);
+    for (; k + 8 <= n; k += 8, e += 256) {
+        int j[8];
+        float2 a[8];
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) j[u] = __ldg(idx + e + 32 * u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) a[u] = make_float2(__ldg(Ah + e + 32 * u), __ldg(Al + e + 32 * u));
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = z[j[u]];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) df_fma1(acc, a[u], v[u]);
+    }
+    for (; k + 4 <= n; k += 4, e += 128) {
+        int j[4];
+        float2 a[4];
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) j[u] = __ldg(idx + e + 32 * u);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] = make_float2(__ldg(Ah + e + 32 * u), __ldg(Al + e + 32 * u));
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = z[j[u]];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) df_fma1(acc, a[u], v[u]);
     }
     for (; k < n; ++k, e += 32) df_fma1(acc, make_float2(__ldg(Ah + e), __ldg(Al + e)), z[__ldg(idx + e)]);
-    return __dadd_rn(__dmul_rn(D.adiag[r], (double)z[r]), df_to_double(acc));
+    zr = (double)zrow;
+    return __dadd_rn(__dmul_rn(D.adiag[r], zr), df_to_double(acc));
 }
 
-// Pass 1's dots with a double-float basis: the block's w and v_j split into
-// (hi, lo) pairs in shared memory, each lane keeps its 8 rows of both in
-// registers; warp `warp` takes basis vectors warp + 8 (4g + u) as in the FP64
-// form, the 8 double-float values of a lane summed across the warp by the
-// same transposing butterfly in double-float, each block's value converted to
-// FP64 once (into dsh) for the FP64 scene sums.
-__device__ __forceinline__ void fg_arn1_dots_df(const Dev& D, float2 wd, float2 vjd, int nv, long r0, int rend,
-                                                double* dsh) {
-    __shared__ float2 wsd[BS_THREADS], vsd[BS_THREADS];
-    wsd[threadIdx.x] = wd;
-    vsd[threadIdx.x] = vjd;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-    constexpr int RPL = BS_THREADS / 32;   // rows per lane
-    const float2* Vb = reinterpret_cast<const float2*>(D.fg_V);
-    for (int base = warp; base < nv; base += 4 * (BS_THREADS / 32)) {
-        // per vector: the lane's 8 rows loaded first, then two accumulation
-        // chains; w and v_j read from shared memory (few registers: the grid
-        // fits the SMs in one wave)
-        float2 x[8];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = base + (BS_THREADS / 32) * u;
-            float2 a = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
-            if (i < nv) {
-                const float2* v = Vb + (long)i * D.fg_ld + r0;
-                float2 vv[RPL];
-#pragma unroll
-                for (int k = 0; k < RPL; ++k) {
-                    const int t = lane + 32 * k;
-                    vv[k] = (r0 + t < rend) ? v[t] : make_float2(0.f, 0.f);
-                }
-#pragma unroll
-                for (int k = 0; k < RPL; ++k) {
-                    const int t = lane + 32 * k;
-                    df_fma(a, vv[k], wsd[t]);
-                    df_fma(c, vv[k], vsd[t]);
-                }
-            }
-            x[2 * u] = a;
-            x[2 * u + 1] = c;
-        }
-        float2 y[4], z[2];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) y[k] = df_add(b4 ? x[k + 4] : x[k], df_shfl_xor(b4 ? x[k] : x[k + 4], 16));
-#pragma unroll
-        for (int k = 0; k < 2; ++k) z[k] = df_add(b3 ? y[k + 2] : y[k], df_shfl_xor(b3 ? y[k] : y[k + 2], 8));
-        float2 tv = df_add(b2 ? z[1] : z[0], df_shfl_xor(b2 ? z[0] : z[1], 4));
-        tv = df_add(tv, df_shfl_xor(tv, 2));
-        tv = df_add(tv, df_shfl_xor(tv, 1));
-        if ((lane & 3) == 0) {
-            const int q = lane >> 2;
-            const int i = base + (BS_THREADS / 32) * (q >> 1);
-            if (i < nv) dsh[(q & 1) ? nv + i : i] = df_to_double(tv);
-        }
+// Pass 1's finisher with the FP64 basis (the scene's last block; tsh: the summed
+// dots h and c): the Gram column and the column's coefficients hc = (2I - Gm) h
+// -- classical Gram-Schmidt applied twice, (I - V V^T)^2 = I - V (2I - V^T V) V^T,
+// with the second projection taken from the Gram matrix instead of a second
+// pass over V.
+__device__ __forceinline__ void fg_arn1_finish(const Dev& D, int s, int j, const double* tsh) {
+    const int nv = j + 1;
+    const FgSmall f = fg_small(D, s);
+    const int ldg = D.fg_m + 1;
+    for (int i = threadIdx.x; i < nv; i += BS_THREADS) {
+        f.Gm[i + (long)j * ldg] = tsh[nv + i];
+        f.Gm[j + (long)i * ldg] = tsh[nv + i];
     }
+    // Gm x for a vector x in shared memory, rows wid, wid + 8, ... by warp, four
+    // rows' loads in flight (Gm is symmetric: row i is read as the contiguous
+    // column i; its new row and column from tsh), the four sums over the lanes by
+    // one transposing butterfly (6 FP64 adds instead of 20: this block's FP64
+    // pipe sets its time); put(i, value) in one lane
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    auto gram = [&](const double* x, auto&& put) {
+        for (int i0 = wid; i0 < nv; i0 += 4 * (BS_THREADS / 32)) {
+            double a[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int k = lane; k < nv; k += 32) {
+                double g[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int i = i0 + u * (BS_THREADS / 32);
+                    g[u] = i >= nv ? 0.0 : i == j ? tsh[nv + k] : k == j ? tsh[nv + i] : __ldcg(f.Gm + (long)i * ldg + k);
+                }
+                const double xk = x[k];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (i0 + u * (BS_THREADS / 32) < nv) a[u] += g[u] * xk;
+            }
+            const bool b4 = lane & 16, b3 = lane & 8;
+            double y[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                y[u] = (b4 ? a[u + 2] : a[u]) + __shfl_xor_sync(0xffffffffu, b4 ? a[u] : a[u + 2], 16);
+            double v = (b3 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b3 ? y[0] : y[1], 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 4);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            const int i = i0 + ((b4 ? 2 : 0) + (b3 ? 1 : 0)) * (BS_THREADS / 32);
+            if ((lane & 7) == 0 && i < nv) put(i, v);
+        }
+    };
+    gram(tsh, [&](int i, double a) {
+        const double acc = 2.0 * tsh[i] - a;
+        f.hc[i] = acc;
+        f.H[i + (long)j * ldg] = acc;
+    });
 }
 
-// Column j, pass 1: w = A z_j (z_j = the V-cycle output in sp2, kept as Z_j;
-// or v_j) into sv; one read of v_0..v_j gives h = V^T w and the Gram column
-// c = V^T v_j.  Finisher: Gm(:,j) = c, then the column's coefficients
-// hc = (2I - Gm) h -- classical Gram-Schmidt applied twice,
-// (I - V V^T)^2 = I - V (2I - V^T V) V^T, with the second projection
-// taken from the Gram matrix instead of a second pass over V.
-template <int DF>
+// Column j, pass 1, FP64 basis: w = A z_j (z_j = the V-cycle output in sp2, kept
+// as Z_j; or v_j) into sv; one read of v_0..v_j gives h = V^T w and the Gram
+// column c = V^T v_j.
 __global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond, int* nconv) {
     BS_PDL_ENTRY();
     const int s = D.blk_scene[blockIdx.x];
-    if (!fg_running(D, s)) {
-        if (DF && (int)blockIdx.x == D.par[s].blk0 && threadIdx.x == 0) D.dyn[s].fg_act = 0;   // no column for pass 2
-        return;
-    }
+    if (!fg_running(D, s)) return;
     const int nact = (D.dyn[s].n + BS_THREADS - 1) / BS_THREADS;
     if ((int)blockIdx.x - D.par[s].blk0 >= nact) return;   // no rows
     __shared__ double ws[BS_THREADS], vs[BS_THREADS];
@@ -1024,29 +1042,15 @@ __global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond, i
     const long col = (long)j * D.fg_ld;
     const double* u = precond ? D.sp2 : D.fg_V + col;
     double w = 0.0, vj = 0.0;
-    float2 vjd = make_float2(0.f, 0.f);
     if (r < rend) {
-        w = DF ? spmv_row_df(D, D.zf, r) : spmv_row64(D, u, r);
+        w = spmv_row64(D, u, r);
         D.sv[r] = w;
-        if (DF) vjd = reinterpret_cast<const float2*>(D.fg_V)[col + r];
-        else vj = D.fg_V[col + r];
+        vj = D.fg_V[col + r];
         if (precond) D.fg_Z[col + r] = D.sp2[r];
     }
-    if (DF) {
-        // u.u for the Gram relation of ||w|| (block partial at dsh[2 nv])
-        __shared__ double wwp[BS_THREADS / 32];
-        const double ww = warp_sum(w * w);
-        if ((threadIdx.x & 31) == 0) wwp[threadIdx.x >> 5] = ww;
-        fg_arn1_dots_df(D, df_split(w), vjd, nv, r0, rend, dsh);
-        if (threadIdx.x == 0) {
-            double a = 0.0;
-            for (int k = 0; k < BS_THREADS / 32; ++k) a += wwp[k];
-            dsh[2 * nv] = a;
-        }
-    } else {
-        ws[threadIdx.x] = w;
-        vs[threadIdx.x] = vj;
-        __syncthreads();
+    ws[threadIdx.x] = w;
+    vs[threadIdx.x] = vj;
+    __syncthreads();
     // Warp w takes basis vectors w + 8 (4g + u), u = 0..3: lanes across the
     // block's rows (coalesced), 8 values per lane (4 vectors x 2 dots), summed
     // over the lanes by a transposing butterfly -- 9 FP64 adds per lane for
@@ -1088,82 +1092,248 @@ __global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond, i
             if (i < nv) dsh[(q & 1) ? nv + i : i] = tv;
         }
     }
+    __syncthreads();
+    if (!fg_scene_sum(D, s, nact, 2 * nv, dsh, tsh, !precond)) return;
+    fg_arn1_finish(D, s, j, tsh);
+}
+
+// Column j, pass 1, double-float basis: w = A z_j for the mixed V-cycle's output
+// (zf; kept as Z_j) into sv, the dots of v_0..v_j with w and v_j, and w.w.
+// Warp w takes the vectors w, w + 8, ...: 8 rows per lane loaded first, then two
+// accumulation chains, w and v_j read from shared memory (48 registers: five
+// blocks per SM).  The dots of four vectors (8 double-float values a lane) are
+// summed over the lanes by a transposing butterfly, w.w of the eight warps by
+// one warp likewise (9 FP64 adds instead of 40), each block's value converted
+// to FP64 once for the FP64 scene sums.  Bound by HBM: 60 us for 313 MB at
+// 0.71 M particles, 0.77 of the measured copy rate.  Measured and not kept: the
+// basis fetched under the SpMV by bulk copies into a ring in shared memory
+// (32 KB and 64 registers: four blocks per SM; 13.86 ms per step against 13.61,
+// 4.20 against 4.06 at 0.18 M).
+__global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1_df(Dev D) {
+    constexpr int NW = BS_THREADS / 32;
+    __shared__ float2 wsd[BS_THREADS], vsd[BS_THREADS];
+    __shared__ double wwp[BS_THREADS];
+    __shared__ double dsh[2 * (BS_FG_MAXM + 1)];
+    __shared__ double tsh[2 * (BS_FG_MAXM + 1)];
+    const int s = D.blk_scene[blockIdx.x];
+    const int blk0 = D.par[s].blk0;
+    const int nact = (D.dyn[s].n + BS_THREADS - 1) / BS_THREADS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // (the scene's state and the basis were written at least two kernels ago)
+    const bool running = fg_running(D, s);
+    if (!running || (int)blockIdx.x - blk0 >= nact) {
+        BS_PDL_ENTRY();
+        return;
+    }
+    const int j = D.dyn[s].fg_j, nv = j + 1;
+    const int rend = D.par[s].row0 + D.dyn[s].n;
+    const long r0 = (long)blockIdx.x * BS_THREADS;
+    const int r = (int)r0 + threadIdx.x;
+    const long col = (long)j * D.fg_ld;
+    const float2* Vb = reinterpret_cast<const float2*>(D.fg_V);
+    const float2 vjd = r < rend ? __ldg(Vb + col + r) : make_float2(0.f, 0.f);
+    BS_PDL_ENTRY();
+    double w = 0.0;
+    if (r < rend) {
+        double zr;
+        w = spmv_row_df(D, D.zf, r, zr);
+        D.sv[r] = w;
+        D.fg_Z[col + r] = zr;
+    }
+    wsd[threadIdx.x] = df_split(w);
+    vsd[threadIdx.x] = vjd;
+    wwp[threadIdx.x] = w * w;
+    __syncthreads();
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    if (warp == NW - 1) {   // w.w: the sums over the lanes of each of the eight warps, then over the warps in order
+        double x[8], y[4], z[2];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = wwp[32 * k + lane];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            y[k] = (b4 ? x[k + 4] : x[k]) + __shfl_xor_sync(0xffffffffu, b4 ? x[k] : x[k + 4], 16);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            z[k] = (b3 ? y[k + 2] : y[k]) + __shfl_xor_sync(0xffffffffu, b3 ? y[k] : y[k + 2], 8);
+        double t = (b2 ? z[1] : z[0]) + __shfl_xor_sync(0xffffffffu, b2 ? z[0] : z[1], 4);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        double a = 0.0;   // warp k's sum is in the lanes 4k .. 4k + 3 (k = 4 b4 + 2 b3 + b2)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a += __shfl_sync(0xffffffffu, t, 4 * k);
+        if (lane == 0) dsh[2 * nv] = a;
+    }
+    for (int base = warp; base < nv; base += 4 * NW) {
+        float2 x[8];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            float2 a = make_float2(0.f, 0.f), c = a;
+            if (base + NW * u < nv) {
+                const float2* v = Vb + (long)(base + NW * u) * D.fg_ld + r0;
+                float2 vv[NW];
+#pragma unroll
+                for (int k = 0; k < NW; ++k) vv[k] = (r0 + lane + 32 * k < rend) ? v[lane + 32 * k] : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < NW; ++k) {
+                    const int t = lane + 32 * k;
+                    df_fma(a, vv[k], wsd[t]);
+                    df_fma(c, vv[k], vsd[t]);
+                }
+            }
+            x[2 * u] = a;
+            x[2 * u + 1] = c;
+        }
+        float2 y[4], z[2];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = df_add(b4 ? x[k + 4] : x[k], df_shfl_xor(b4 ? x[k] : x[k + 4], 16));
+#pragma unroll
+        for (int k = 0; k < 2; ++k) z[k] = df_add(b3 ? y[k + 2] : y[k], df_shfl_xor(b3 ? y[k] : y[k + 2], 8));
+        float2 tv = df_add(b2 ? z[1] : z[0], df_shfl_xor(b2 ? z[0] : z[1], 4));
+        tv = df_add(tv, df_shfl_xor(tv, 2));
+        tv = df_add(tv, df_shfl_xor(tv, 1));
+        if ((lane & 3) == 0) {
+            const int qq = lane >> 2;
+            const int i = base + NW * (qq >> 1);
+            if (i < nv) dsh[(qq & 1) ? nv + i : i] = df_to_double(tv);
+        }
     }
     __syncthreads();
-    if (!fg_scene_sum(D, s, nact, DF ? 2 * nv + 1 : 2 * nv, dsh, tsh, !precond)) return;
-    const FgSmall f = fg_small(D, s);
-    const int ldg = D.fg_m + 1;
-    for (int i = threadIdx.x; i < nv; i += BS_THREADS) {
-        f.Gm[i + (long)j * ldg] = tsh[nv + i];
-        f.Gm[j + (long)i * ldg] = tsh[nv + i];
+    fg_group_sum(D, s, nact, 2 * nv + 1, dsh, tsh, wwp);   // (the scene's sums and the coefficients: k_fg_fin)
+}
+
+// The scene's sums and the column's coefficients with the double-float basis,
+// one cluster of BS_FIN_BLOCKS blocks per scene (one block took 30 us of the
+// 90 of pass 1 at 0.71 M particles: an FP64 instruction of a warp holds the
+// SM's FP64 pipe for 16 cycles, and its loads came one chain after another).
+// Each block sums its share of the 2 nv + 1 values over the groups (every
+// sub-sum a thread's) and sends them to the others; the rows of the Gram
+// products are shared out likewise, their old part loaded into registers before
+// the wait for pass 1.  The orders of all sums are those of fg_sum_rows and of
+// a warp per row.
+//   hc = (2I - Gm) h (fg_arn1_finish), and h_{j+1,j} = ||w|| for w = u - V c
+// without a pass over w: ||w||^2 = u.u - 2 c.h + c^T Gm c (u = A z_j, h = V^T u,
+// Gm = V^T V, c = hc), so pass 2 can write v_{j+1} and the V-cycle input
+// directly.  When that difference falls below 1e-6 u.u the estimate is not
+// trusted and the cycle restarts from the true residual.  Pass 2 also runs the
+// column's rotations (in a block of its own, beside the streaming ones).
+#define BS_FIN_BLOCKS 8
+__global__ void __launch_bounds__(BS_THREADS) k_fg_fin(Dev D) {
+    constexpr int NB = BS_FIN_BLOCKS, NV = BS_FG_MAXM + 1;
+    constexpr int RW = (NV + 8 * NB - 1) / (8 * NB), KL = (NV + 31) / 32;   // rows per warp, values per lane
+    __shared__ double tot[2 * NV + 1], hcs[NV], gts[NV], eparts[8];
+    __shared__ double scr[4 * BS_THREADS / NB + 4 * BS_THREADS], scr2[BS_THREADS / NB + BS_THREADS];
+    const int s = blockIdx.x / NB, rank = (int)cluster_rank(), t = threadIdx.x;
+    const int lane = t & 31, wid = t >> 5;
+    SceneDyn& Y = D.dyn[s];
+    if (!fg_running(D, s)) {   // (the state was written at least two kernels ago)
+        BS_PDL_ENTRY();
+        if (rank == 0 && t == 0) Y.fg_act = 0;   // no column for pass 2
+        return;
     }
-    // Gm x for a vector x in shared memory, rows wid, wid + 8, ... by warp, four
-    // rows' loads in flight (Gm is symmetric: row i is read as the contiguous
-    // column i; its new row and column from tsh), the four sums over the lanes by
-    // one transposing butterfly (6 FP64 adds instead of 20: this block's FP64
-    // pipe sets its time); put(i, value) in one lane
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const ScenePar& P = D.par[s];
+    const FgSmall f = fg_small(D, s);
+    const int j = Y.fg_j, nv = j + 1, nvals = 2 * nv + 1;
+    const int ldg = D.fg_m + 1, ld = bs::fg_part_ld(D.fg_m);
+    const int cnt = (P.nblk + 31) >> 5, have = ((Y.n + BS_THREADS - 1) / BS_THREADS + 31) >> 5;
+    // this warp's rows of Gm: rank + NB (wid + 8 m); its new row and column come with the sums
+    double g[RW][KL];
+#pragma unroll
+    for (int m = 0; m < RW; ++m) {
+        const int i = rank + NB * (wid + 8 * m);
+#pragma unroll
+        for (int c = 0; c < KL; ++c) {
+            const int k = lane + 32 * c;
+            g[m][c] = i < j && k < j ? __ldcg(f.Gm + (long)i * ldg + k) : 0.0;
+        }
+    }
+    cluster_arrive();   // every block of the cluster runs before remote stores
+    BS_PDL_ENTRY();
+    // this block's values [v0, v0 + nmine)
+    const int per = (nvals + NB - 1) / NB, v0 = rank * per, nmine = max(0, min(per, nvals - v0));
+    const double* __restrict__ src = D.fg_gpart + (long)P.grp0 * ld + v0;
+    const int Q = nvals <= BS_THREADS ? BS_THREADS / nvals : 1;   // sub-sums of a value (rows q, q + Q, ...)
+    const int A = nvals <= BS_THREADS ? 4 : 2;                    // accumulators of a sub-sum
+    for (int e = t; e < nmine * Q * A; e += BS_THREADS) {
+        const int i = e % nmine, qa = e / nmine, q = qa % Q, u = qa / Q;
+        const int m = cnt > q ? (cnt - q + Q - 1) / Q : 0, full = m / A * A;
+        const int mh = have > q ? (have - q + Q - 1) / Q : 0;
+        double a = 0.0;
+        for (int k0 = u; k0 < min(mh, full); k0 += 8 * A) {
+            double v[8];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) v[x] = k0 + x * A < min(mh, full) ? __ldcg(src + (long)(q + (k0 + x * A) * Q) * ld + i) : 0.0;
+#pragma unroll
+            for (int x = 0; x < 8; ++x)
+                if (k0 + x * A < min(mh, full)) a += v[x];
+        }
+        if (u == 0)
+            for (int k = full; k < mh; ++k) a += __ldcg(src + (long)(q + k * Q) * ld + i);
+        scr[e] = a;
+    }
+    __syncthreads();
+    for (int e = t; e < nmine * Q; e += BS_THREADS) {
+        const int st = nmine * Q;
+        scr2[e] = A == 4 ? (scr[e] + scr[e + st]) + (scr[e + 2 * st] + scr[e + 3 * st]) : scr[e] + scr[e + st];
+    }
+    cluster_wait();
+    __syncthreads();
+    if (t < nmine) {
+        double a = 0.0;
+        if (A == 4)
+            for (int q = 0; q < Q; ++q) a += scr2[q * nmine + t];
+        else
+            a = scr2[t];
+        const unsigned p = (unsigned)__cvta_generic_to_shared(tot + v0 + t);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) st_rank(p, b, a);
+    }
+    cluster_arrive();
+    cluster_wait();
+    // Gm x for a vector x in shared memory, one row after another of this warp
     auto gram = [&](const double* x, auto&& put) {
-        for (int i0 = wid; i0 < nv; i0 += 4 * (BS_THREADS / 32)) {
-            double a[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int k = lane; k < nv; k += 32) {
-                double g[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int i = i0 + u * (BS_THREADS / 32);
-                    g[u] = i >= nv ? 0.0 : i == j ? tsh[nv + k] : k == j ? tsh[nv + i] : __ldcg(f.Gm + (long)i * ldg + k);
-                }
-                const double xk = x[k];
+        for (int m = 0; m < RW; ++m) {
+            const int i = rank + NB * (wid + 8 * m);
+            if (i >= nv) break;
+            double a = 0.0;
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (i0 + u * (BS_THREADS / 32) < nv) a[u] += g[u] * xk;
+            for (int c = 0; c < KL; ++c) {
+                const int k = lane + 32 * c;
+                if (k < nv) a += (i == j ? tot[nv + k] : k == j ? tot[nv + i] : g[m][c]) * x[k];
             }
-            const bool b4 = lane & 16, b3 = lane & 8;
-            double y[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-                y[u] = (b4 ? a[u + 2] : a[u]) + __shfl_xor_sync(0xffffffffu, b4 ? a[u] : a[u + 2], 16);
-            double v = (b3 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b3 ? y[0] : y[1], 8);
-            v += __shfl_xor_sync(0xffffffffu, v, 4);
-            v += __shfl_xor_sync(0xffffffffu, v, 2);
-            v += __shfl_xor_sync(0xffffffffu, v, 1);
-            const int i = i0 + ((b4 ? 2 : 0) + (b3 ? 1 : 0)) * (BS_THREADS / 32);
-            if ((lane & 7) == 0 && i < nv) put(i, v);
+            a = warp_sum(a);
+            put(i, a);
         }
     };
-    // hc = (2I - Gm) h
-    __shared__ double hcs[BS_FG_MAXM + 1];
-    gram(tsh, [&](int i, double a) {
-        const double acc = 2.0 * tsh[i] - a;
-        f.hc[i] = acc;
-        f.H[i + (long)j * ldg] = acc;
-        hcs[i] = acc;
+    gram(tot, [&](int i, double a) {
+        const double acc = 2.0 * tot[i] - a;
+        if (lane < NB) st_rank((unsigned)__cvta_generic_to_shared(hcs + i), lane, acc);
+        if (lane == 0) {
+            f.hc[i] = acc;
+            f.H[i + (long)j * ldg] = acc;
+            f.Gm[i + (long)j * ldg] = tot[nv + i];
+            f.Gm[j + (long)i * ldg] = tot[nv + i];
+        }
     });
-    if (!DF) return;
-    // h_{j+1,j} = ||w|| for w = u - V c without a pass over w: ||w||^2 =
-    // u.u - 2 c.h + c^T Gm c (u = A z_j, h = V^T u, Gm = V^T V, c = hc), so
-    // pass 2 can write v_{j+1} and the V-cycle input directly.  When that
-    // difference falls below 1e-6 u.u the estimate is not trusted and the
-    // cycle restarts from the true residual.  Pass 2 also runs the column's
-    // rotations (in a block of its own, beside the streaming ones).
-    __shared__ double eparts[BS_THREADS / 32];
-    __syncthreads();
-    // (a warp's rows in order, then the warps)
-    __shared__ double gts[BS_FG_MAXM + 1];
-    gram(hcs, [&](int i, double g) { gts[i] = g; });
-    __syncwarp();
-    if (lane == 0) {
+    cluster_arrive();
+    cluster_wait();
+    gram(hcs, [&](int i, double a) {
+        if (lane == 0) st_rank((unsigned)__cvta_generic_to_shared(gts + i), 0, a);
+    });
+    cluster_arrive();
+    cluster_wait();
+    if (rank != 0) return;
+    if (t < 8) {   // the rows t, t + 8, ... in order, then these sums in order
         double part = 0.0;
-        for (int i = wid; i < nv; i += BS_THREADS / 32) part += hcs[i] * (gts[i] - 2.0 * tsh[i]);
-        eparts[wid] = part;
+        for (int i = t; i < nv; i += 8) part += hcs[i] * (gts[i] - 2.0 * tot[i]);
+        eparts[t] = part;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const double uu = tsh[2 * nv];
+    if (t == 0) {
+        const double uu = tot[2 * nv];
         double eta2 = uu;
-        for (int w = 0; w < BS_THREADS / 32; ++w) eta2 += eparts[w];
+        for (int w = 0; w < 8; ++w) eta2 += eparts[w];
         const double hn = sqrt(fmax(eta2, 0.0));
-        SceneDyn& Y = D.dyn[s];
         Y.fg_c = j;
         Y.fg_hn = hn;
         Y.fg_bad = !(eta2 > 1e-6 * uu);
@@ -1309,6 +1479,27 @@ __global__ void k_fg_update(Dev D, int precond) {
 
 namespace bs {
 
+// pass 1 of a column with the double-float basis: the row blocks, then the
+// scenes' clusters
+static void fg_pass1_df(const Dev& D, const Launch& L) {
+    launch_pdl(L, k_fg_arn1_df, L.nblk_rows, BS_THREADS, 0, D);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(D.nscene * BS_FIN_BLOCKS));
+    cfg.blockDim = dim3(BS_THREADS);
+    cfg.stream = L.stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = BS_FIN_BLOCKS;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, k_fg_fin, D);
+    *L.launches += 1;
+}
+
 // Host driver of the FP64 solve.  Checks the converged-scene counter every
 // `check_every` iterations with one event sync, one chunk behind the launches
 // so the GPU never idles on the host.
@@ -1426,10 +1617,10 @@ void solve_fgmres(const Dev& D, const Launch& L, int maxit, int check_every, int
     };
     auto column = [&]() {
         if (!D.fg_df) put();
-        if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.sp2, 1);
+        if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.fg_df ? nullptr : D.sp2, 1);   // (pass 1 of the double-float form reads zf)
         int q2 = tbegin(L, K_FG_ARN);
-        if (D.fg_df) launch_pdl(L, k_fg_arn1<1>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
-        else launch_pdl(L, k_fg_arn1<0>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
+        if (D.fg_df) fg_pass1_df(D, L);
+        else launch_pdl(L, k_fg_arn1, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
         tend(L, q2);
         q2 = tbegin(L, K_FG_ORTH);
         if (D.fg_df) launch_pdl(L, k_fg_arn2<1>, L.nblk_rows + D.nscene, BS_THREADS, 0, D, d_nconv, mgmode);
@@ -1649,10 +1840,10 @@ void fg_put(const Dev& D, const Launch& L, int mgmode) {
 
 void fg_column(const Dev& D, const Launch& L, int precond, int mg_prec, int mgmode, int* d_nconv) {
     if (!D.fg_df) fg_put(D, L, mgmode);
-    if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.sp2, 1);
+    if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.fg_df ? nullptr : D.sp2, 1);   // (pass 1 of the double-float form reads zf)
     int q = tbegin(L, K_FG_ARN);
-    if (D.fg_df) launch_pdl(L, k_fg_arn1<1>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
-    else launch_pdl(L, k_fg_arn1<0>, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
+    if (D.fg_df) fg_pass1_df(D, L);
+    else launch_pdl(L, k_fg_arn1, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
     tend(L, q);
     q = tbegin(L, K_FG_ORTH);
     if (D.fg_df) launch_pdl(L, k_fg_arn2<1>, L.nblk_rows + D.nscene, BS_THREADS, 0, D, d_nconv, mgmode);
