@@ -189,6 +189,17 @@ class Context:
         """Scene s's particle fields in the library's row order.  out: a dict
         from pinned_state() (or a previous download) to fill instead of new
         arrays; the result is views of its first n rows."""
+        if out is not None:   # the library reports the count: no query before the read-back
+            keys = abi.STATE_FIELDS_F64 + abi.STATE_FIELDS_I32 + ["flags"]
+            keys += abi.EXTRA_F64 + ["coff", "cell"] if full else []
+            rows = min(len(out[k]) if k in out else 0 for k in keys)
+            if rows:
+                st, res = abi.state_out(rows, full, out)
+                rc = lib.bs_download(self.h, s, C.byref(st))
+                if rc == 0:
+                    return {k: v[:st.n] for k, v in res.items()}
+                if rc != abi.BS_E_CAPACITY:
+                    self._check(rc, "download")
         n = self.info(s)["n"]
         st, res = abi.state_out(n, full, out)
         self._check(lib.bs_download(self.h, s, C.byref(st)), "download")

@@ -373,6 +373,36 @@ __global__ void k_upload_gather(Dev D, int row0, int n, int cell0, int has_flags
     D.cell[r] = D.cell2[g] / 2 + cell0;
 }
 
+// The scene's rows of the requested fields straight into the caller's page-locked
+// buffers, with its dynamic state (one launch instead of a copy per field: a
+// small scene's read-back is bound by the copies' launches).  Nothing is written
+// where the scene has more rows than the buffers (n_out; the caller reads the
+// count from the dynamic state).
+__global__ void k_read_back(const __grid_constant__ bs::SnapArgs a, const SceneDyn* dyn, SceneDyn* dyn_out,
+                            const int* cell, int cell0, int* cell_dst, const double* c0, const double* c1,
+                            const double* c2, const double* c3, double* coff_dst) {
+    const int n = dyn->n;
+    if (blockIdx.x == 0)
+        for (int e = threadIdx.x; e < (int)(sizeof(SceneDyn) / sizeof(int)); e += blockDim.x)
+            ((int*)dyn_out)[e] = ((const int*)dyn)[e];
+    if (n > a.n) return;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int r = a.row0 + q;
+#pragma unroll 4
+    for (int f = 0; f < a.nf; ++f) a.dst[f][q] = a.src[f][r];
+    if (a.tid) a.tid_dst[q] = a.tid[r];
+    if (a.pid) a.pid_dst[q] = a.pid[r];
+    if (a.flags) a.flags_dst[q] = a.flags[r];
+    if (cell_dst) cell_dst[q] = cell[r] - cell0;
+    if (coff_dst) {
+        coff_dst[4 * (size_t)q] = c0[r];
+        coff_dst[4 * (size_t)q + 1] = c1[r];
+        coff_dst[4 * (size_t)q + 2] = c2[r];
+        coff_dst[4 * (size_t)q + 3] = c3[r];
+    }
+}
+
 // Rows [row0, row0 + n) of the requested fields into the snapshot buffer
 // (same row positions), one launch in stream order after a step: the copy
 // to the host then reads the snapshot while the next steps run.
@@ -583,6 +613,14 @@ void cell_max_timestep(const Dev& D, const Launch& L, int do_cellmax, int do_tim
 void advance_time(const Dev& D, const Launch& L) {
     const int q = tbegin(L, K_ADVANCE);
     k_advance_time<<<gdiv(D.nscene, 64), 64, 0, L.stream>>>(D);
+    tend(L, q);
+}
+
+void read_back(const Dev& D, const Launch& L, const SnapArgs& a, int s, int rows, SceneDyn* dyn_out, int cell0,
+               int* cell_dst, double* coff_dst) {
+    const int q = tbegin(L, K_DERIVE);
+    k_read_back<<<gdiv(rows > 0 ? rows : 1, BS_THREADS), BS_THREADS, 0, L.stream>>>(
+        a, D.dyn + s, dyn_out, D.cell, cell0, cell_dst, D.c0, D.c1, D.c2, D.c3, coff_dst);
     tend(L, q);
 }
 

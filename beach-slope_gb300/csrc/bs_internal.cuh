@@ -708,6 +708,9 @@ struct SnapArgs {
     uint8_t* flags_dst;
 };
 void snapshot(const Launch& L, const SnapArgs& a);
+// the same rows (a.n: the buffers' rows) straight into page-locked host buffers, with the dynamic state (k_read_back)
+void read_back(const Dev& D, const Launch& L, const SnapArgs& a, int s, int rows, SceneDyn* dyn_out, int cell0,
+               int* cell_dst, double* coff_dst);
 // an uploaded scene's rows into their binned order (see k_upload_gather)
 void upload_gather(const Dev& D, const Launch& L, int row0, int n, int cell0, int has_flags, int has_pid);
 // solver
