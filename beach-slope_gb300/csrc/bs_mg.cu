@@ -150,25 +150,26 @@ __global__ void k_mg_galc(Dev D, int l) {
     const int nyf = M.ny[l][s], nxf = M.nx[l][s], fo = M.off[l][s];
     const T* Af = (const T*)M.A[l];
     const int nf = M.n[l];
+    // the four children's stencils, all loads before the sums; entry k of child
+    // (a, b) falls on one entry of the coarse stencil
+    T v[4][9];
+#pragma unroll
+    for (int ch = 0; ch < 4; ++ch) {
+        const int fi = 2 * I + (ch & 1), fj = 2 * J + (ch >> 1);
+        const bool in = fi < nyf && fj < nxf;
+        const int c = fo + fj * nyf + fi;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v[ch][k] = in ? Af[(long)k * nf + c] : (T)0;
+    }
     double acc[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) acc[k] = 0.0;
-    for (int b = 0; b < 2; ++b)
-        for (int a = 0; a < 2; ++a) {
-            const int fi = 2 * I + a, fj = 2 * J + b;
-            if (fi >= nyf || fj >= nxf) continue;
-            const int c = fo + fj * nyf + fi;
 #pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                const double v = (double)Af[(long)k * nf + c];
-                if (v == 0.0) continue;
-                const int ni = fi + (k % 3) - 1, nj = fj + (k / 3) - 1;
-                const int ci = (ni >= 0 ? ni / 2 : -1) - I, cj = (nj >= 0 ? nj / 2 : -1) - J;
-                const int t = (cj + 1) * 3 + (ci + 1);
+    for (int ch = 0; ch < 4; ++ch)
 #pragma unroll
-                for (int u = 0; u < 9; ++u)
-                    if (u == t) acc[u] += v;
-            }
+        for (int k = 0; k < 9; ++k) {
+            const int ci = ((ch & 1) + k % 3 + 1) / 2 - 1, cj = ((ch >> 1) + k / 3 + 1) / 2 - 1;   // -1, 0 or 1
+            if (v[ch][k] != (T)0) acc[(cj + 1) * 3 + ci + 1] += (double)v[ch][k];
         }
     T* Ac = (T*)M.A[l + 1];
     const int nc = M.n[l + 1];
@@ -678,18 +679,21 @@ __global__ void __launch_bounds__(BS_CHIP_THREADS) k_mg_chip_pack(Dev D, __grid_
             const int jl = chip_div(e, invy), i = e - jl * sy - 1, j = L.j0 - 1 + jl;
             DV[e] = (i >= 0 && i < L.ny && j >= 0 && j < L.nx && jl <= L.nc + 1) ? dv[j * L.ny + i] : (T)0;
         }
-        for (int q = t; q < L.Q; q += BS_CHIP_THREADS) {
+        for (int e = t; e < 4 * L.Q; e += BS_CHIP_THREADS) {   // a thread per child
+            const int q = e >> 2, ch = e & 3;
             int I, J;
             const uint2 w = chip_quad(L, sizeof(T), q, &I, &J);
-            ((uint2*)(cst + L.tab))[q] = w;
-            for (int ch = 0; ch < 4; ++ch) {
-                const int i = 2 * I + (ch & 1), j = L.j0 + 2 * J + (ch >> 1);
-                for (int s = 0; s < 9; ++s) {
-                    const int ni = i + (s % 3) - 1, nj = j + (s / 3) - 1;
-                    const bool in = (w.y >> ch & 1) && !(ni < 0 || nj < 0 || ni >= L.ny || nj >= L.nx);
-                    ((T*)(cst + L.A))[(s * L.Q + q) * 4 + ch] = in ? A[s * n + j * L.ny + i] : (T)0;
-                }
+            if (ch == 0) ((uint2*)(cst + L.tab))[q] = w;
+            const int i = 2 * I + (ch & 1), j = L.j0 + 2 * J + (ch >> 1);
+            T v[9];
+#pragma unroll
+            for (int s = 0; s < 9; ++s) {
+                const int ni = i + (s % 3) - 1, nj = j + (s / 3) - 1;
+                const bool in = (w.y >> ch & 1) && !(ni < 0 || nj < 0 || ni >= L.ny || nj >= L.nx);
+                v[s] = in ? A[s * n + j * L.ny + i] : (T)0;
             }
+#pragma unroll
+            for (int s = 0; s < 9; ++s) ((T*)(cst + L.A))[(s * L.Q + q) * 4 + ch] = v[s];
         }
     }
 }

@@ -1436,15 +1436,38 @@ __global__ void k_fg_solve(Dev D, int* nconv) {
     const int k = Y.fg_j;
     const int ld = D.fg_m + 1;
     const FgSmall f = fg_small(D, s);
-    for (int i = k - 1; i >= 0; --i) {
-        double acc = 0.0;
-        for (int l = i + 1 + lane; l < k; l += 32) acc += f.H[i + (long)l * ld] * ys[l];
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            const double d = f.H[i + (long)i * ld];
-            ys[i] = d != 0.0 ? (f.g[i] - acc) / d : 0.0;
+    // row i's entries right of the diagonal (lane: i + 1 + lane, + 32, ...), loaded a row ahead: a row
+    // needs nothing of the one before it but its y
+    constexpr int PER = (BS_FG_MAXM + 31) / 32;
+    double h[PER], hn[PER], d = 0.0, g = 0.0, dn, gn;
+    auto row = [&](int i, double (&v)[PER], double& di, double& gi) {
+#pragma unroll
+        for (int c = 0; c < PER; ++c) {
+            const int l = i + 1 + lane + 32 * c;
+            v[c] = i >= 0 && l < k ? __ldcg(f.H + i + (long)l * ld) : 0.0;
         }
+        di = i >= 0 ? __ldcg(f.H + i + (long)i * ld) : 0.0;
+        gi = i >= 0 ? __ldcg(f.g + i) : 0.0;
+    };
+    row(k - 1, h, d, g);
+    for (int i = k - 1; i >= 0; --i) {
+        row(i - 1, hn, dn, gn);
+        double acc = 0.0;
+#pragma unroll
+        for (int c = 0; c < PER; ++c) {
+            const int l = i + 1 + lane + 32 * c;
+            if (l < k) acc += h[c] * ys[l];
+        }
+        // the sum over the lanes; the first k - 1 - i hold terms, the others 0
+        const int terms = k - 1 - i;
+        for (int o = 16; o > 0; o >>= 1)
+            if (terms > o) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) ys[i] = d != 0.0 ? (g - acc) / d : 0.0;
         __syncwarp();
+        d = dn;
+        g = gn;
+#pragma unroll
+        for (int c = 0; c < PER; ++c) h[c] = hn[c];
     }
     for (int i = lane; i < k; i += 32) f.y[i] = ys[i];
     if (lane == 0) {
