@@ -532,12 +532,12 @@ __global__ void k_true_res64(Dev D) {
 //
 // Two forms of a column.  FP64 basis (fg_df = 0): k_fg_put writes v_j and the
 // V-cycle input, pass 1 (k_fg_arn1) the SpMV and the dots, pass 2
-// (k_fg_arn2<0>) the projection, the norm and, in its finisher, the
+// (k_fg_arn2) the projection, the norm and, in its finisher, the
 // rotations.  Double-float basis (fg_df = 1, the preconditioned mixed solve):
 // the basis is stored as (hi, lo) FP32 pairs and its dots and projection run
 // on the FP32 pipe; pass 1 (k_fg_arn1_df) also sums u.u and its finisher takes
 // h_{j+1,j} from the Gram relation and runs the rotations, so pass 2
-// (k_fg_arn2<1>) streams v_{j+1} and the next V-cycle input with no reduction
+// (k_fg_arn2_df) streams v_{j+1} and the next V-cycle input with no reduction
 // and k_fg_put runs once per cycle.
 
 // Per-scene small storage: H [(m+1) x m] column-major (R of the rotated
@@ -1342,60 +1342,22 @@ __global__ void __launch_bounds__(BS_THREADS) k_fg_fin(Dev D) {
     }
 }
 
-// Column j, pass 2: w -= V hc (the pending vector, into ss), h_{j+1,j} = ||w||;
-// finisher: rotations, residual estimate, cycle end
-// With the double-float basis (DF): column j = fg_j - 1 was finished by pass
-// 1, and this pass writes v_{j+1} = (w - V hc) / h_{j+1,j} into the basis
-// and the V-cycle input (mgmode as k_fg_put), with no reduction.
-// Its first D.nscene blocks (DF) run the scenes' rotations (fg_finish_column),
-// beside the streaming blocks; these read only what pass 1 left (fg_c, fg_act,
-// fg_rinv), so a cycle that ends with this column has one vector too many.
-template <int DF>
+// Column j, pass 2, FP64 basis: w -= V hc (the pending vector, into ss),
+// h_{j+1,j} = ||w||; finisher: rotations, residual estimate, cycle end
 __global__ void k_fg_arn2(Dev D, int* nconv, int mgmode) {
     BS_PDL_ENTRY();
-    if (DF && (int)blockIdx.x < D.nscene) {
-        const SceneDyn& Y = D.dyn[blockIdx.x];
-        if (Y.fg_act) fg_finish_column(D, blockIdx.x, fg_small(D, blockIdx.x), Y.fg_c, Y.fg_hn, Y.fg_bad != 0, false, nconv);
-        return;
-    }
-    const int blk = DF ? blockIdx.x - D.nscene : blockIdx.x;
-    const int s = D.blk_scene[blk];
-    if (DF ? !D.dyn[s].fg_act : !fg_running(D, s)) return;
+    const int s = D.blk_scene[blockIdx.x];
+    if (!fg_running(D, s)) return;
     __shared__ double hs[BS_FG_MAXM + 1];
-    __shared__ float2 hsd[BS_FG_MAXM + 1];
     const ScenePar& P = D.par[s];
-    const int j = DF ? D.dyn[s].fg_c : D.dyn[s].fg_j;
+    const int j = D.dyn[s].fg_j;
     const int rend = P.row0 + D.dyn[s].n;
-    const int r = blk * blockDim.x + threadIdx.x;
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const FgSmall f = fg_small(D, s);
-    for (int i = threadIdx.x; i <= j; i += BS_THREADS) {
-        hs[i] = f.hc[i];
-        if (DF) hsd[i] = df_split(hs[i]);
-    }
+    for (int i = threadIdx.x; i <= j; i += BS_THREADS) hs[i] = f.hc[i];
     __syncthreads();
     double q[1] = {0.0};
-    if (DF) {   // w -= (V hc) summed in double-float, then v_{j+1}
-        if (r >= rend) return;
-        double w = D.sv[r];
-        const float2* v = reinterpret_cast<const float2*>(D.fg_V) + r;
-        const long ld = D.fg_ld;
-        float2 a0 = make_float2(0.f, 0.f), a1 = a0, a2 = a0, a3 = a0;
-        int i = 0;
-        for (; i + 4 <= j + 1; i += 4) {   // four loads in flight, four chains
-            const float2 v0 = v[i * ld], v1 = v[(i + 1) * ld], v2 = v[(i + 2) * ld], v3 = v[(i + 3) * ld];
-            df_fma(a0, hsd[i], v0);
-            df_fma(a1, hsd[i + 1], v1);
-            df_fma(a2, hsd[i + 2], v2);
-            df_fma(a3, hsd[i + 3], v3);
-        }
-        for (; i <= j; ++i) df_fma(a0, hsd[i], v[i * ld]);
-        w = __dsub_rn(w, df_to_double(df_add(df_add(a0, a1), df_add(a2, a3))));
-        const double vn = w * D.dyn[s].fg_rinv;
-        reinterpret_cast<float2*>(D.fg_V)[(long)(j + 1) * ld + r] = df_split(vn);
-        if (mgmode == 1) bs::mg_put_input<double>(D, r, vn);
-        else if (mgmode == 2) bs::mg_put_input<float>(D, r, vn);
-        return;
-    } else if (r < rend) {
+    if (r < rend) {
         double w = D.sv[r];
         const double* v = D.fg_V + r;
         int i = 0;
@@ -1419,7 +1381,88 @@ __global__ void k_fg_arn2(Dev D, int* nconv, int mgmode) {
         D.dyn[s].fg_rinv = hns > 0.0 ? 1.0 / hns : 0.0;
     }
     __syncthreads();
-    fg_finish_column(D, s, f, j, hns, false, mgmode == 0, nconv);   // (a preconditioned solve keeps the plain chain)
+    // (a preconditioned solve keeps the plain chain)
+    fg_finish_column(D, s, f, j, hns, false, mgmode == 0, nconv);
+}
+
+// Column j, pass 2, double-float basis: v_{j+1} = (w - V hc) / h_{j+1,j} into
+// the basis, and the V-cycle input (mgmode as k_fg_put), with no reduction.  Two
+// rows per thread (16-byte loads of the basis), eight vectors in flight; per
+// row four sums, the vectors in turn.  The first D.nscene blocks run the scenes'
+// rotations (fg_finish_column) beside the streaming blocks; these read only
+// what k_fg_fin left (fg_c, fg_act, fg_rinv), so a cycle that ends with this
+// column has one vector too many.
+#define BS_ARN2_THREADS (BS_ALIGN / 2)
+__global__ void __launch_bounds__(BS_ARN2_THREADS) k_fg_arn2_df(Dev D, int* nconv, int mgmode) {
+    BS_PDL_ENTRY();
+    if ((int)blockIdx.x < D.nscene) {
+        const SceneDyn& Y = D.dyn[blockIdx.x];
+        if (Y.fg_act) fg_finish_column(D, blockIdx.x, fg_small(D, blockIdx.x), Y.fg_c, Y.fg_hn, Y.fg_bad != 0, false, nconv);
+        return;
+    }
+    const int blk = blockIdx.x - D.nscene;
+    const int s = D.blk_scene[blk];
+    if (!D.dyn[s].fg_act) return;
+    __shared__ float2 hsd[BS_FG_MAXM + 1];
+    const int j = D.dyn[s].fg_c;
+    const int rend = D.par[s].row0 + D.dyn[s].n;
+    const int r = blk * BS_ALIGN + 2 * threadIdx.x;
+    const FgSmall f = fg_small(D, s);
+    for (int i = threadIdx.x; i <= j; i += BS_ARN2_THREADS) hsd[i] = df_split(f.hc[i]);
+    __syncthreads();
+    if (r >= rend) return;
+    const double rinv = D.dyn[s].fg_rinv;
+    const double2 w2 = *reinterpret_cast<const double2*>(D.sv + r);
+    const long ld = D.fg_ld / 2;
+    const float4* v = reinterpret_cast<const float4*>(D.fg_V) + r / 2;   // (x, y): the first row, (z, w): the second
+    float2 a[4], b[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) a[c] = b[c] = make_float2(0.f, 0.f);
+    int i = 0;
+    for (; i + 8 <= j + 1; i += 8) {
+        float4 x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = v[(i + u) * ld];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const float2 h = hsd[i + u];
+            df_fma(a[u & 3], h, make_float2(x[u].x, x[u].y));
+            df_fma(b[u & 3], h, make_float2(x[u].z, x[u].w));
+        }
+    }
+    {   // the last ones: four in turn, then the rest into the first sum
+        float4 x[7];
+        const int left = j + 1 - i;
+#pragma unroll
+        for (int u = 0; u < 7; ++u) x[u] = u < left ? v[(i + u) * ld] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 7; ++u) {
+            if (u >= left) break;
+            const float2 h = hsd[i + u];
+            const float2 p = make_float2(x[u].x, x[u].y), q = make_float2(x[u].z, x[u].w);
+            if (u < 4 && left >= 4) {
+                df_fma(a[u], h, p);
+                df_fma(b[u], h, q);
+            } else {
+                df_fma(a[0], h, p);
+                df_fma(b[0], h, q);
+            }
+        }
+    }
+    const double vn0 = __dsub_rn(w2.x, df_to_double(df_add(df_add(a[0], a[1]), df_add(a[2], a[3])))) * rinv;
+    const double vn1 = __dsub_rn(w2.y, df_to_double(df_add(df_add(b[0], b[1]), df_add(b[2], b[3])))) * rinv;
+    const float2 s0 = df_split(vn0), s1 = df_split(vn1);
+    float2* out = reinterpret_cast<float2*>(D.fg_V) + (long)(j + 1) * D.fg_ld + r;
+    auto put = [&](int q, double x) {
+        if (mgmode == 1) bs::mg_put_input<double>(D, q, x);
+        else if (mgmode == 2) bs::mg_put_input<float>(D, q, x);
+    };
+    out[0] = s0;
+    put(r, vn0);
+    if (r + 1 < rend) {
+        out[1] = s1;
+        put(r + 1, vn1);
+    }
 }
 
 // One warp per scene: y = R^-1 g over the cycle's k columns; scenes that
@@ -1646,8 +1689,8 @@ void solve_fgmres(const Dev& D, const Launch& L, int maxit, int check_every, int
         else launch_pdl(L, k_fg_arn1, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
         tend(L, q2);
         q2 = tbegin(L, K_FG_ORTH);
-        if (D.fg_df) launch_pdl(L, k_fg_arn2<1>, L.nblk_rows + D.nscene, BS_THREADS, 0, D, d_nconv, mgmode);
-        else launch_pdl(L, k_fg_arn2<0>, L.nblk_rows, BS_THREADS, 0, D, d_nconv, mgmode);
+        if (D.fg_df) launch_pdl(L, k_fg_arn2_df, L.nblk_rows + D.nscene, BS_ARN2_THREADS, 0, D, d_nconv, mgmode);
+        else launch_pdl(L, k_fg_arn2, L.nblk_rows, BS_THREADS, 0, D, d_nconv, mgmode);
         tend(L, q2);
     };
     IterGraph* G = L.graph;
@@ -1869,8 +1912,8 @@ void fg_column(const Dev& D, const Launch& L, int precond, int mg_prec, int mgmo
     else launch_pdl(L, k_fg_arn1, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
     tend(L, q);
     q = tbegin(L, K_FG_ORTH);
-    if (D.fg_df) launch_pdl(L, k_fg_arn2<1>, L.nblk_rows + D.nscene, BS_THREADS, 0, D, d_nconv, mgmode);
-    else launch_pdl(L, k_fg_arn2<0>, L.nblk_rows, BS_THREADS, 0, D, d_nconv, mgmode);
+    if (D.fg_df) launch_pdl(L, k_fg_arn2_df, L.nblk_rows + D.nscene, BS_ARN2_THREADS, 0, D, d_nconv, mgmode);
+    else launch_pdl(L, k_fg_arn2, L.nblk_rows, BS_THREADS, 0, D, d_nconv, mgmode);
     tend(L, q);
 }
 
