@@ -403,6 +403,18 @@ void fill_par(ScenePar& P, const bs_params& p, int kmax) {
     P.kq_lam_h = (float)P.lam;
     P.kq_lam_l = (float)(P.lam - (double)P.kq_lam_h);
     P.kq_pad = 0.0f;
+    P.f_h = (float)P.h;
+    P.f_hl = (float)(P.h - (double)P.f_h);
+    P.f_ih = (float)P.inv_h;
+    P.f_ihl = (float)(P.inv_h - (double)P.f_ih);
+    P.f_ih2 = (float)P.inv_h2;
+    P.f_ih3 = (float)P.inv_h3;
+    P.f_cn1 = (float)P.cn1;
+    P.f_cn2 = (float)P.cn2;
+    P.f_twoh = (float)P.twoh;
+    P.f_twoh2 = (float)(P.twoh * P.twoh);
+    P.f_cw = (float)P.cw;
+    P.f_pad = 0.0f;
     P.rho = p.rho; P.rhomin = p.rhomin; P.rhomax = p.rhomax; P.rel_den = p.rel_den; P.g = p.g;
     P.mu = p.mu; P.tschmidt = p.tschmidt; P.por = p.por; P.lamk = p.lamk; P.d50 = p.d50;
     P.freethr = p.lamfs * p.maxdivr; P.csh = p.csh; P.maxshift = p.maxshift; P.sig1 = p.sig1;
@@ -656,7 +668,7 @@ int bs_create(int32_t nscenes, const bs_params* params, const int32_t* capacity,
         A(scan_part, (size_t)mc * nscenes);
     }
     A(gx, (size_t)gr); A(gy, (size_t)gr); A(gv, (size_t)gr); A(gcell_start, C); A(gcell_end, C);
-    A(gxr, (size_t)gr); A(gyr, (size_t)gr); A(gpos4, (size_t)gr); A(xr, R); A(yr, R);
+    A(gxr, (size_t)gr + BS_CAND); A(gyr, (size_t)gr + BS_CAND); A(gpos4, (size_t)gr); A(xyr, R + BS_CAND);
     if (ctx->precision == BS_PREC_MIXED) {
         A(pos4, R); A(rec0, R); A(rec1, R); A(rec2, R); A(volf2, R); A(cfa, R); A(cfb, R);
     }

@@ -22,6 +22,7 @@
 
 #define BS_ALIGN 256
 #define BS_THREADS 256
+#define BS_CAND 8   // candidates the neighbour search loads at once (up to this many past the last row)
 #define BS_NCAT 10      // bucket categories per cell in the re-bin (see k_rank)
 #define BS_MAXDOT 8     // partial sums per block in the solver
 #define BS_SCAN_CHUNK 1024  // cells per block of the re-bin's cell scan
@@ -56,6 +57,9 @@ struct ScenePar {                 // per-scene constants
     // the kernel gradient on the FP32 pipe as F = kq_s g(q), q = r/h:
     // kq_s = fl32(cn1/h^2), (hi, lo) pairs of cn2/cn1, 3 (1 + cn2/cn1) and lam
     float kq_s, kq_rho_h, kq_rho_l, kq_k3_h, kq_k3_l, kq_lam_h, kq_lam_l, kq_pad;
+    // FP32 roundings of the constants above (a conversion in a kernel holds the
+    // FP64 pipe as long as 60 FP32 instructions), h and 1/h as (hi, lo)
+    float f_h, f_hl, f_ih, f_ihl, f_ih2, f_ih3, f_cn1, f_cn2, f_twoh, f_twoh2, f_cw, f_pad;
 };
 
 struct SceneDyn {                 // per-scene dynamic state (device)
@@ -139,7 +143,7 @@ struct MgExact {
 struct Dev {
     // particle fields (current buffer)
     double *x, *y, *xs, *ys, *vx, *vy, *vxs, *vys, *p, *mass, *rho, *oden, *ovol, *con;
-    float *xr, *yr;                 // position relative to the row's cell corner (xleft, ybot), FP32
+    float2* xyr;                    // position relative to the row's cell corner (xleft, ybot), FP32
     float4* pos4;                   // mixed: position as (x hi, x lo, y hi, y lo) FP32 pairs (f2_split2),
                                     // written by k_relpos and by the packs of the sweeps that read it (k_quot)
     double *vol, *nu;               // derived: m/rho, vis(oden)/oden
@@ -261,12 +265,12 @@ struct KerF {
 };
 __device__ __forceinline__ KerF ker_f(const ScenePar& P) {
     KerF K;
-    K.h = (float)P.h;
-    K.ih = (float)P.inv_h;
-    K.ih2 = (float)P.inv_h2;
-    K.ih3 = (float)P.inv_h3;
-    K.c1 = (float)P.cn1;
-    K.c2 = (float)P.cn2;
+    K.h = P.f_h;
+    K.ih = P.f_ih;
+    K.ih2 = P.f_ih2;
+    K.ih3 = P.f_ih3;
+    K.c1 = P.f_cn1;
+    K.c2 = P.f_cn2;
     return K;
 }
 __device__ __forceinline__ float bs_Wf(float r, const KerF& K) {
@@ -416,7 +420,6 @@ __device__ __forceinline__ void f2_acc_prod(float2& a, float2 k, float rh, float
     a.x = t.x;
     a.y = __fadd_rn(a.y, __fadd_rn(t.y, te));
 }
-
 // Radial factor F(r) of the hybrid-kernel gradient: grad_i W_ij = F(r) (r_i - r_j)
 // (kernel.f90:94-162: Wabx(p1=j, p2=i) = F * (p2%x - p1%x)).
 __device__ __forceinline__ double bs_F(double r, const ScenePar& P) {

@@ -15,41 +15,45 @@ struct RowCtx {
     bool held;     // a particle row of a held scene
 };
 
-__device__ __forceinline__ RowCtx row_ctx(const Dev& D) {
+__device__ __forceinline__ RowCtx row_ctx(const Dev& D, unsigned block) {
     RowCtx c;
-    c.r = blockIdx.x * blockDim.x + threadIdx.x;
+    c.r = block * blockDim.x + threadIdx.x;
     c.s = D.blk_scene[c.r / BS_ALIGN];   // the block's scene, whatever the block size
     const bool row = c.r < D.par[c.s].row0 + D.dyn[c.s].n;
     c.held = row && D.dyn[c.s].hold;
     c.active = row && !c.held;
     return c;
 }
+__device__ __forceinline__ RowCtx row_ctx(const Dev& D) { return row_ctx(D, blockIdx.x); }
 
 // The four cells of the quadrant stencil in the reference's order
 // (search.f90:328-388): cell q lies (di0 + (q & 1), dj0 + (q >> 1)) rows and
 // columns from the row's cell c, i.e. at c + dj celly + di.  ordp packs
 // effpor's order of the same four (porous.f90:125-176: the row's own cell,
 // then the other three of the quadrant as listed), two bits per entry.
-// False for a non-finite position.
-__device__ __forceinline__ bool quad_cells(const ScenePar& P, int c, double xi, double yi, int& di0, int& dj0,
-                                          int& ordp) {
-    const int lc = c - P.cell0;
-    const int i = lc % P.celly + 1, j = lc / P.celly + 1;
-    const double xl = cell_xleft(P, j), xr = cell_xright(P, j);
-    const double yb = cell_ybot(P, i), yt = cell_ytop(P, i);
-    const double mx = xl + fabs((xl - xr) / 2.0);
-    const double my = yb + fabs((yt - yb) / 2.0);
-    if (xi <= mx && yi <= my) {
-        di0 = 0; dj0 = -1; ordp = 2 | 0 << 2 | 3 << 4 | 1 << 6;
-    } else if (xi > mx && yi <= my) {
-        di0 = 0; dj0 = 0; ordp = 0 | 2 << 2 | 1 << 4 | 3 << 6;
-    } else if (xi > mx && yi > my) {
-        di0 = -1; dj0 = 0; ordp = 1 | 2 << 2 | 0 << 4 | 3 << 6;
-    } else if (xi <= mx && yi > my) {
-        di0 = -1; dj0 = -1; ordp = 3 | 2 << 2 | 0 << 4 | 1 << 6;
-    } else {
-        return false;
+// False for a non-finite position.  The halves are told apart by the FP32
+// position in the cell (k_relpos: within 1e-7 of its size) away from the middle,
+// 2h, and by the reference's FP64 expressions near it: those are 25 of the
+// search's 150 FP64 instructions, which hold the SM's pipe for 16 cycles each.
+__device__ __forceinline__ bool quad_cells(const ScenePar& P, int c, double xi, double yi, float2 rel, int& di0,
+                                          int& dj0, int& ordp) {
+    const float mid = P.f_twoh;
+    bool right = rel.x > mid, up = rel.y > mid;
+    if (!(fabsf(rel.x - mid) > 1e-5f * mid && fabsf(rel.y - mid) > 1e-5f * mid)) {
+        const int lc = c - P.cell0;
+        const int i = lc % P.celly + 1, j = lc / P.celly + 1;
+        const double xl = cell_xleft(P, j), xr = cell_xright(P, j);
+        const double yb = cell_ybot(P, i), yt = cell_ytop(P, i);
+        const double mx = xl + fabs((xl - xr) / 2.0);
+        const double my = yb + fabs((yt - yb) / 2.0);
+        right = xi > mx;
+        up = yi > my;
+        if (!(right || xi <= mx) || !(up || yi <= my)) return false;
     }
+    di0 = up ? -1 : 0;
+    dj0 = right ? 0 : -1;
+    ordp = up ? (right ? 1 | 2 << 2 | 0 << 4 | 3 << 6 : 3 | 2 << 2 | 0 << 4 | 1 << 6)
+              : (right ? 0 | 2 << 2 | 1 << 4 | 3 << 6 : 2 | 0 << 2 | 3 << 4 | 1 << 6);
     return true;
 }
 
@@ -72,8 +76,7 @@ __global__ void k_relpos(Dev D) {
     const int lc = D.cell[r] - P.cell0;
     const int i = lc % P.celly + 1, j = lc / P.celly + 1;
     const double x = D.x[r], y = D.y[r];
-    D.xr[r] = (float)(x - cell_xleft(P, j));
-    D.yr[r] = (float)(y - cell_ybot(P, i));
+    D.xyr[r] = make_float2((float)(x - cell_xleft(P, j)), (float)(y - cell_ybot(P, i)));
     if (P.precision == BS_PREC_MIXED) {
         D.pos4[r] = f2_split2(x, y);
         D.volf2[r] = f2_split(D.vol[r]);
@@ -85,11 +88,37 @@ __device__ __forceinline__ T ld(const void* p, long e) { return ((const T*)p)[e]
 template <typename T>
 __device__ __forceinline__ void st(void* p, long e, T v) { ((T*)p)[e] = v; }
 
+// 2^-60 <= v < 2^50 (or v = +0), by the words
+__device__ __forceinline__ bool in_range(double v, bool zero = false) {
+    const int hi = __double2hiint(v);
+    return (hi >= (1023 - 60) << 20 && hi < (1023 + 50) << 20) || (zero && (hi | __double2loint(v)) == 0);
+}
+
 // ------------------------------------------------------------------ search
-// nsearch2 (search.f90:13-308) and effpor/porsearch (porous.f90:32-224)
+// nsearch2 (search.f90:13-308) and effpor/porsearch (porous.f90:32-224).
+//
+// Bound by instruction issue at large sizes (70% of the slots; 12,000
+// instructions per warp, half of them the pairs' double-float arithmetic; FP64
+// pipe 30%) and by the latency of a row's chain at small ones.  So the two
+// halves, which share nothing but the row, run in blocks of their own,
+// interleaved (an FP64-heavy and an FP32-heavy warp beside each other: with all
+// of one half first 539 instead of 504 us at 1.04 M rows); BS_CAND candidates
+// are loaded at once and their tests become bit masks (no branch per candidate;
+// the next batch's loads ahead cost more instructions than the wait: 531 instead
+// of 463 us); 64 registers (four blocks of 256: 72 costs 3% at 1 M rows, 48
+// spills); scene constants are rounded to FP32 on the host.  Packed FP32 instructions
+// for two pairs at once gave nothing (439 and 439 us).
+// Both halves at 15 k, 187 k, 712 k and 1.04 M rows (64 scenes), before and now:
+// 64 and 32, 163 and 102, 382 and 293, 510 and 437 us; FP64 at 187 k 675 and
+// 616 us (IEEE divisions and roots on the FP64 pipe).
 template <typename T>
-__global__ void __launch_bounds__(BS_THREADS) k_search(Dev D, int do_search, int do_effpor) {
-    const RowCtx R = row_ctx(D);
+__global__ void __launch_bounds__(BS_THREADS, 4) k_search(Dev D, int do_search, int do_effpor) {
+    unsigned block = blockIdx.x;
+    if (do_search && do_effpor) {
+        (block & 1 ? do_search : do_effpor) = 0;
+        block >>= 1;
+    }
+    const RowCtx R = row_ctx(D, block);
     if (!R.active) {
         if (R.held && do_effpor) {   // keep a held scene's density across the buffer swap
             D.rho_new[R.r] = D.rho[R.r];
@@ -103,8 +132,9 @@ __global__ void __launch_bounds__(BS_THREADS) k_search(Dev D, int do_search, int
     const double xi = D.x[r], yi = D.y[r];
     const int c = D.cell[r];
     int di0, dj0, ordp;
-    const bool ok = quad_cells(P, c, xi, yi, di0, dj0, ordp);
-    const float cwf = (float)P.cw;
+    const float2 rel = D.xyr[r];
+    const bool ok = quad_cells(P, c, xi, yi, rel, di0, dj0, ordp);
+    const float cwf = P.f_cw;
     uint8_t fl = D.flags[r];
     if (do_search) {
         const int kmax = D.kmax;
@@ -114,38 +144,59 @@ __global__ void __launch_bounds__(BS_THREADS) k_search(Dev D, int do_search, int
         // error of d^2 below 2e-6 relative for coordinates within a cell) --
         // outside [lo, hi] the exact FP64 test cannot disagree -- and the
         // exact test of functions.f90:38 / search.f90:59 (IEEE sqrt, no FMA,
-        // FP64 positions) inside it.  Only indices are appended, so the
-        // warp's divergence is cheap.
-        const float t2f = (float)(twoh * twoh);
+        // FP64 positions) inside it.  Only indices are appended, by predicated
+        // stores.
+        constexpr int NB = BS_CAND;   // candidates in flight
+        const float t2f = P.f_twoh2;
         const float thr_hi = t2f * (1.0f + 1e-5f), thr_lo = t2f * (1.0f - 1e-5f);
         int cnt = 0;
-        auto test = [&](int rj, float fx, float fy) {
-            const float d2f = fx * fx + fy * fy;
-            if (d2f > thr_hi) return;
-            if (d2f >= thr_lo) {
-                const double dx = __ldg(D.x + rj) - xi, dy = __ldg(D.y + rj) - yi;
-                const double rad = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-                if (!(rad < twoh)) return;
-            }
-            if (cnt < kmax) D.nidx[ell(r, cnt, kmax)] = rj;
-            ++cnt;
-        };
         if (ok) {
-            const float xri = D.xr[r], yri = D.yr[r];
+            const float2 nrel = make_float2(-rel.x, -rel.y);
+            int first[4], last[4];
+#pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int di = di0 + (q & 1), dj = dj0 + (q >> 1);
-                const int cq = c + dj * P.celly + di;
-                float ox, oy;
-                cell_offset(cwf, dj, di, ox, oy);
-                const int r1 = D.cell_end[cq];
-                int rj = D.cell_start[cq];
-                for (; rj + 1 < r1; rj += 2) {   // two independent candidate loads in flight
-                    const float x0 = __ldg(D.xr + rj) + ox, y0 = __ldg(D.yr + rj) + oy;
-                    const float x1 = __ldg(D.xr + rj + 1) + ox, y1 = __ldg(D.yr + rj + 1) + oy;
-                    if (rj != r) test(rj, x0 - xri, y0 - yri);   // (tid, matid) self-exclusion
-                    if (rj + 1 != r) test(rj + 1, x1 - xri, y1 - yri);
+                const int cq = c + (dj0 + (q >> 1)) * P.celly + di0 + (q & 1);
+                first[q] = D.cell_start[cq];
+                last[q] = D.cell_end[cq];
+            }
+            int* out = D.nidx + ell(r, 0, kmax);
+#pragma unroll 1
+            for (int q = 0; q < 4; ++q) {
+                float2 off;
+                cell_offset(cwf, dj0 + (q >> 1), di0 + (q & 1), off.x, off.y);
+                const int r1 = q == 0 ? last[0] : q == 1 ? last[1] : q == 2 ? last[2] : last[3];
+#pragma unroll 1
+                for (int rj = q == 0 ? first[0] : q == 1 ? first[1] : q == 2 ? first[2] : first[3]; rj < r1; rj += NB) {
+                    // (the array runs NB past the last row: what lies past r1 is masked)
+                    const float2* const from = D.xyr + rj;
+                    float2 at[NB];
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) at[k] = __ldg(from + k);
+                    unsigned in = 0, edge = 0;
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) {
+                        const float2 f = __fadd2_rn(__fadd2_rn(at[k], off), nrel);
+                        const float d2f = f.x * f.x + f.y * f.y;
+                        if (!(d2f > thr_hi)) in |= 1u << k;
+                        if (d2f >= thr_lo) edge |= 1u << k;
+                    }
+                    in &= ((1u << BS_CAND) - 1) >> max(NB - (r1 - rj), 0);
+                    const unsigned self = (unsigned)(r - rj);   // (tid, matid) self-exclusion
+                    if (self < NB) in &= ~(1u << self);
+                    edge &= in;
+                    for (; edge; edge &= edge - 1) {
+                        const int k = __ffs(edge) - 1;
+                        const double dx = __ldg(D.x + rj + k) - xi, dy = __ldg(D.y + rj + k) - yi;
+                        const double rad = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+                        if (!(rad < twoh)) in &= ~(1u << k);
+                    }
+#pragma unroll
+                    for (int k = 0; k < NB; ++k)
+                        if (in >> k & 1) {
+                            if (cnt < kmax) out[32 * cnt] = rj + k;
+                            ++cnt;
+                        }
                 }
-                if (rj < r1 && rj != r) test(rj, (__ldg(D.xr + rj) + ox) - xri, (__ldg(D.yr + rj) + oy) - yri);
             }
         }
         if (cnt > kmax) set_err(D, R.s, BS_ERR_NBR_OVERFLOW);
@@ -182,13 +233,21 @@ __global__ void __launch_bounds__(BS_THREADS) k_search(Dev D, int do_search, int
             float2 s00 = make_float2(0.f, 0.f), s01 = s00, s10 = s00, s11 = s00;
             const float kqs = P.kq_s;
             const float2 kr = make_float2(P.kq_rho_h, P.kq_rho_l), k3 = make_float2(P.kq_k3_h, P.kq_k3_l);
-            const float2 hf = f2_split(P.h), ihd = f2_split(P.inv_h);
+            const float2 hf = make_float2(P.f_h, P.f_hl), ihd = make_float2(P.f_ih, P.f_ihl);
             const float2 lam = make_float2(P.kq_lam_h, P.kq_lam_l);
             const float4 pi4 = D.pos4[r];
-            for (int k = 0; k < n; ++k) {
+            // the next pair's position and volume and the index after it in flight
+            const int* const list = D.nidx + ell(r, 0, kmax);
+            const int end = max(n - 1, 0);
+            int rn = n > 0 ? list[0] : r;
+            float4 pj4 = __ldg(D.pos4 + rn), pn4 = pj4;
+            float2 vj = __ldg(D.volf2 + rn), vn = vj;
+            rn = n > 0 ? list[32 * min(1, end)] : r;
+            for (int k = 0; k < n; ++k, pj4 = pn4, vj = vn) {
                 const long e = ell(r, k, kmax);
-                const int rj = D.nidx[e];
-                const float4 pj4 = __ldg(D.pos4 + rj);
+                pn4 = __ldg(D.pos4 + rn);
+                vn = __ldg(D.volf2 + rn);
+                rn = list[32 * min(k + 2, end)];
                 const float2 dx = f2_diff(pj4.x, pj4.y, pi4.x, pi4.y);
                 const float2 dy = f2_diff(pj4.z, pj4.w, pi4.z, pi4.w);
                 const PairR pr = pair_r(dx, dy);
@@ -218,7 +277,6 @@ __global__ void __launch_bounds__(BS_THREADS) k_search(Dev D, int do_search, int
                 st<T>(D.nkx, e, (T)kx);
                 st<T>(D.nky, e, (T)ky);
                 // V (dx hi + dx lo) as (hi, lo) from V as (hi, lo)
-                const float2 vj = __ldg(D.volf2 + rj);
                 const float r1h = __fmul_rn(vj.x, dx.x);
                 const float r1e = __fmaf_rn(vj.y, dx.x, __fmaf_rn(vj.x, dx.y, __fmaf_rn(vj.x, dx.x, -r1h)));
                 const float r3h = __fmul_rn(vj.x, dy.x);
@@ -291,15 +349,16 @@ __global__ void __launch_bounds__(BS_THREADS) k_search(Dev D, int do_search, int
         double phi = 1.0, res = 0.0;
         if (tid == BS_TID_FLUID) {
             double sf = 0.0;
+            bool clear = sizeof(T) == 4;   // mixed: no grain within 2h
             if (ok) {
                 // effpor's cell order (porous.f90:125-176): its own cell, then
                 // the other three of the same quadrant in the listed order
                 const double wsolid = 1.0 - P.por * 1.0;
-                const float wsf = (float)wsolid, t2c = (float)(P.twoh * P.twoh);
+                const float wsf = (float)wsolid, t2c = P.f_twoh2;
                 Kahan32 sff;
                 const KerF KF = ker_f(P);
-                const float t2f = (float)(P.twoh * P.twoh) * (1.0f + 1e-5f);
-                const float xri = D.xr[r], yri = D.yr[r];
+                constexpr int NG = BS_CAND;   // grains in flight
+                const float t2f = t2c * (1.0f + 1e-5f);
                 float4 pi4 = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (sizeof(T) == 4) pi4 = D.pos4[r];
                 for (int k = 0; k < 4; ++k) {
@@ -309,40 +368,67 @@ __global__ void __launch_bounds__(BS_THREADS) k_search(Dev D, int do_search, int
                     float ox, oy;
                     cell_offset(cwf, dj, di, ox, oy);
                     const int g1 = D.gcell_end[cq];
-                    for (int g = D.gcell_start[cq]; g < g1; ++g) {
+                    for (int g0 = D.gcell_start[cq]; g0 < g1; g0 += NG) {
                         // FP32 prefilter (as in the neighbour scan): a grain
                         // rejected here is outside 2h in FP64 as well
-                        const float fx = (__ldg(D.gxr + g) + ox) - xri, fy = (__ldg(D.gyr + g) + oy) - yri;
-                        if (fx * fx + fy * fy > t2f) continue;
-                        if (sizeof(T) == 4) {
-                            // mixed: FP32 (W(2h) = 0: the cut needs no exact
-                            // test), the offset from the double-float positions
-                            const float4 g4 = __ldg(D.gpos4 + g);
-                            const float ex = f2_diff(pi4.x, pi4.y, g4.x, g4.y).x;
-                            const float ey = f2_diff(pi4.z, pi4.w, g4.z, g4.w).x;
-                            const float s2 = ex * ex + ey * ey;
-                            if (s2 < t2c) {
-                                float rad = 0.0f;   // grains may coincide with pore particles
-                                if (s2 > 0.0f) {
-                                    float ir = rsqrtf(s2);
-                                    ir = ir * (1.5f - 0.5f * s2 * ir * ir);
-                                    rad = s2 * ir;
+                        // (the arrays run NG past the last grain, as the rows')
+                        const float *const fx0 = D.gxr + g0, *const fy0 = D.gyr + g0;
+                        float xs[NG], ys[NG];
+#pragma unroll
+                        for (int m = 0; m < NG; ++m) {
+                            xs[m] = __ldg(fx0 + m);
+                            ys[m] = __ldg(fy0 + m);
+                        }
+                        unsigned in = 0;
+#pragma unroll
+                        for (int m = 0; m < NG; ++m) {
+                            const float fx = (xs[m] + ox) - rel.x, fy = (ys[m] + oy) - rel.y;
+                            if (!(fx * fx + fy * fy > t2f)) in |= 1u << m;
+                        }
+                        in &= ((1u << BS_CAND) - 1) >> max(NG - (g1 - g0), 0);
+                        for (; in; in &= in - 1) {
+                            const int g = g0 + __ffs(in) - 1;
+                            if (sizeof(T) == 4) {
+                                // mixed: FP32 (W(2h) = 0: the cut needs no exact
+                                // test), the offset from the double-float positions
+                                const float4 g4 = __ldg(D.gpos4 + g);
+                                const float ex = f2_diff(pi4.x, pi4.y, g4.x, g4.y).x;
+                                const float ey = f2_diff(pi4.z, pi4.w, g4.z, g4.w).x;
+                                const float s2 = ex * ex + ey * ey;
+                                if (s2 < t2c) {
+                                    float rad = 0.0f;   // grains may coincide with pore particles
+                                    if (s2 > 0.0f) {
+                                        float ir = rsqrtf(s2);
+                                        ir = ir * (1.5f - 0.5f * s2 * ir * ir);
+                                        rad = s2 * ir;
+                                    }
+                                    sff.add(wsf * bs_Wf(rad, KF) * (float)D.gv[g]);
                                 }
-                                sff.add(wsf * bs_Wf(rad, KF) * (float)D.gv[g]);
+                            } else {
+                                const double dx = xi - D.gx[g], dy = yi - D.gy[g];
+                                const double rad = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+                                if (rad < P.twoh) sf = sf + wsolid * bs_W(rad, P) * D.gv[g];
                             }
-                        } else {
-                            const double dx = xi - D.gx[g], dy = yi - D.gy[g];
-                            const double rad = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-                            if (rad < P.twoh) sf = sf + wsolid * bs_W(rad, P) * D.gv[g];
                         }
                     }
                 }
-                if (sizeof(T) == 4) sf = sff.value();
+                if (sizeof(T) == 4) {
+                    clear = sff.s == 0.0f && sff.c == 0.0f;
+                    if (!clear) sf = sff.value();
+                }
             }
-            if (sf > (1.0 - P.por)) sf = 1.0 - P.por;
-            phi = 1.0 - sf;
-            const double od = D.oden[r];
-            const double rn = phi * od;
+            const double od = D.oden[r], vx = D.vx[r], vy = D.vy[r];
+            // Clear of grains phi is 1 and both drag terms end in a product with
+            // 1 - phi = +0 (-0 - 0 in all): for values whose other factors are
+            // finite the 70 FP64 instructions are left out (tested on the
+            // words: a comparison in FP64 holds the pipe, too).
+            clear = clear && in_range(od) && in_range(fabs(vx), true) && in_range(fabs(vy), true) &&
+                    in_range(P.lamk, true) && in_range(P.d50) && in_range(P.por) && __double2hiint(P.por) < 0x3ff00000;
+            if (!clear) {
+                if (sf > (1.0 - P.por)) sf = 1.0 - P.por;
+                phi = 1.0 - sf;
+            }
+            const double rn = clear ? od : phi * od;
             if (do_effpor == 2) {   // WCSPH: the density is the continuity equation's
                 D.rho_new[r] = D.rho[r];
                 D.vol_new[r] = D.vol[r];
@@ -350,26 +436,29 @@ __global__ void __launch_bounds__(BS_THREADS) k_search(Dev D, int do_search, int
                 D.rho_new[r] = rn;
                 D.vol_new[r] = sizeof(T) == 4 ? D.mass[r] * fast_rcp64(rn) : D.mass[r] / rn;
             }
-            const double phi3 = phi * phi * phi;
-            const double vx = D.vx[r], vy = D.vy[r];
-            if (sizeof(T) == 4) {
-                // mixed: the same drag with Newton-step reciprocals and square
-                // roots (~1e-13 relative) in place of IEEE division and sqrt
-                double sp3, isp3, vm = 0.0, slk = 0.0, t;
-                fast_r64(150.0 * phi3, t, isp3);
-                const double Fch = 1.750 * isp3;
-                fast_r64(phi3, sp3, t);
-                const double v2 = vx * vx + vy * vy;
-                if (v2 > 0.0) fast_r64(v2, vm, t);
-                if (P.lamk > 0.0) fast_r64(P.lamk, slk, t);
-                const double om = 1.0 - phi;
-                res = -(bs_vis(od) * fast_rcp64(od) * P.lamk * (om * om) * fast_rcp64(phi3 * (P.d50 * P.d50))) -
-                      (Fch * vm * slk * om * fast_rcp64(sp3 * P.d50));
+            if (clear) {
+                res = -0.0;
             } else {
-                const double Fch = 1.750 / sqrt(150.0 * phi3);
-                const double vm = sqrt(vx * vx + vy * vy);
-                res = -((bs_vis(od) / od) * P.lamk * ((1.0 - phi) * (1.0 - phi)) / (phi3 * (P.d50 * P.d50))) -
-                      ((Fch * vm * sqrt(P.lamk) * (1.0 - phi)) / (sqrt(phi3) * P.d50));
+                const double phi3 = phi * phi * phi;
+                if (sizeof(T) == 4) {
+                    // mixed: the same drag with Newton-step reciprocals and square
+                    // roots (~1e-13 relative) in place of IEEE division and sqrt
+                    double sp3, isp3, vm = 0.0, slk = 0.0, t;
+                    fast_r64(150.0 * phi3, t, isp3);
+                    const double Fch = 1.750 * isp3;
+                    fast_r64(phi3, sp3, t);
+                    const double v2 = vx * vx + vy * vy;
+                    if (v2 > 0.0) fast_r64(v2, vm, t);
+                    if (P.lamk > 0.0) fast_r64(P.lamk, slk, t);
+                    const double om = 1.0 - phi;
+                    res = -(bs_vis(od) * fast_rcp64(od) * P.lamk * (om * om) * fast_rcp64(phi3 * (P.d50 * P.d50))) -
+                          (Fch * vm * slk * om * fast_rcp64(sp3 * P.d50));
+                } else {
+                    const double Fch = 1.750 / sqrt(150.0 * phi3);
+                    const double vm = sqrt(vx * vx + vy * vy);
+                    res = -((bs_vis(od) / od) * P.lamk * ((1.0 - phi) * (1.0 - phi)) / (phi3 * (P.d50 * P.d50))) -
+                          ((Fch * vm * sqrt(P.lamk) * (1.0 - phi)) / (sqrt(phi3) * P.d50));
+                }
             }
         } else {
             D.rho_new[r] = D.rho[r];
@@ -1600,7 +1689,12 @@ __global__ void __launch_bounds__(BS_THREADS) k_ghost(Dev D, int use_mls) {
 
 void search(const Dev& D, const Launch& L, int precision, int do_search, int do_effpor) {
     BS_PLAIN(K_RELPOS, k_relpos, D);
-    BS_DISPATCH(K_SEARCH, precision, k_search, D, do_search, do_effpor);
+    // the two halves in blocks of their own where both run
+    const unsigned grid = row_blocks(L, L.sweep_tpb) * (do_search && do_effpor ? 2 : 1);
+    const int q = tbegin(L, K_SEARCH);
+    if (precision == BS_PREC_MIXED) k_search<float><<<grid, L.sweep_tpb, 0, L.stream>>>(D, do_search, do_effpor);
+    else k_search<double><<<grid, L.sweep_tpb, 0, L.stream>>>(D, do_search, do_effpor);
+    tend(L, q);
 }
 void freesurf(const Dev& D, const Launch& L) { BS_PLAIN(K_FREESURF, k_freesurf, D); }
 void eddy(const Dev& D, const Launch& L, int precision, int with_eddy, int with_varts, int with_disp) {
