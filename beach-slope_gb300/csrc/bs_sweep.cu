@@ -485,12 +485,24 @@ __global__ void k_freesurf(Dev D) {
     }
 }
 
+// The mixed sweeps below are bound by the latency of a neighbour's chain (its
+// index from HBM or L2, then its records: 35 of 42 cycles between a warp's
+// instructions), so each loads a batch of B neighbours' pair data and then their
+// records before the first pair's arithmetic, which stays in list order.  B is
+// what the registers allow: one more and the lost warps cost more than the loads
+// gain (comp_vel at B = 3, 4, 6: 101, 91, 97 us per launch with its k_quot at
+// 1.04 M rows; k_eddy 136, 128, 128).  Before and now at 187 k and 1.04 M rows
+// (launches with their k_quot averaged): eddy 31 and 29, 140 and 124 us; int_vel
+// 51 and 40, 222 and 171; scalar 47 and 32, 162 and 125; comp_vel 26 and 26, 111
+// and 91; assembly 59 and 45 us at 187 k (712 k: 145 and 150, bound by HBM there).
+// k_shift and the WCSPH continuity gained nothing and keep one neighbour at a time.
+
 // ------------------------------------------------------------------ eddyvis
 // turbulence.f90:12-113, with int_vel's varts (integrator.f90:468-507: the
 // same L-corrected velocity-gradient sums) and optionally the per-particle
 // dispersion tensor used by the next scalar sub-steps (scalar.f90:276-301).
 template <typename T>
-__global__ void __launch_bounds__(BS_THREADS) k_eddy(Dev D, int with_eddy, int with_varts, int with_disp) {
+__global__ void __launch_bounds__(BS_THREADS, sizeof(T) == 4 ? 5 : 1) k_eddy(Dev D, int with_eddy, int with_varts, int with_disp) {
     const RowCtx R = row_ctx(D);
     if (!R.active) return;
     const ScenePar& P = D.par[R.s];
@@ -515,17 +527,34 @@ __global__ void __launch_bounds__(BS_THREADS) k_eddy(Dev D, int with_eddy, int w
         // from the k_quot records, the differences rounded once to FP32
         const float4 q4 = D.rec0[r];
         const CorrF cf = corr_f(D, r);
-        for (int k = 0; k < n; ++k) {
-            const long e = ell(r, k, kmax);
-            const int j = D.nidx[e];
-            const float z1 = ld<float>(D.nkx, e), z2 = ld<float>(D.nky, e);
-            const float4 qj = __ldg(D.rec0 + j);
-            const float a = f2_diff(qj.x, qj.y, q4.x, q4.y).x, b = f2_diff(qj.z, qj.w, q4.z, q4.w).x;
-            const float V = __ldg(D.rec1 + j).x;
-            const float Lx = cf.lx(z1, z2), Ly = cf.ly(z1, z2);
-            t1 += V * a * Lx;
-            t2 += V * b * Ly;
-            t3 += 0.5f * V * (a * Ly + b * Lx);
+        constexpr int B = 4;   // (48 registers, five blocks of 256: 128 us without the bound, 124 with it)
+        for (int k0 = 0; k0 < n; k0 += B) {
+            int js[B];
+            float z1s[B], z2s[B], Vs[B];
+            float4 qs[B];
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                const long e = ell(r, min(k0 + m, n - 1), kmax);
+                js[m] = D.nidx[e];
+                z1s[m] = ld<float>(D.nkx, e);
+                z2s[m] = ld<float>(D.nky, e);
+            }
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                qs[m] = __ldg(D.rec0 + js[m]);
+                Vs[m] = __ldg(D.rec1 + js[m]).x;
+            }
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                if (k0 + m >= n) break;
+                const float z1 = z1s[m], z2 = z2s[m], V = Vs[m];
+                const float4 qj = qs[m];
+                const float a = f2_diff(qj.x, qj.y, q4.x, q4.y).x, b = f2_diff(qj.z, qj.w, q4.z, q4.w).x;
+                const float Lx = cf.lx(z1, z2), Ly = cf.ly(z1, z2);
+                t1 += V * a * Lx;
+                t2 += V * b * Ly;
+                t3 += 0.5f * V * (a * Ly + b * Lx);
+            }
         }
     }
     for (int k = 0; k < (sizeof(T) == 4 ? 0 : n); ++k) {
@@ -604,43 +633,66 @@ __global__ void __launch_bounds__(BS_THREADS) k_intvel(Dev D) {
         const KerF KF = ker_f(P);
         const CorrF cf = corr_f(D, r);
         Kahan32 kx, ky;
-        for (int k = 0; k < n; ++k) {
-            const long e = ell(r, k, kmax);
-            const int j = D.nidx[e];
-            const float z1 = ld<float>(D.nkx, e), z2 = ld<float>(D.nky, e);
-            const float pd = ld<float>(D.nrinv, e);
-            const int tj = D.tid[j];
-            const float4 kj = __ldg(D.rec1 + j), wj = __ldg(D.rec2 + j);
-            float cmu;
-            if (tj == BS_TID_FLUID) {   // harmonic mean
-                const float nuj = kj.w;
-                cmu = 2.0f * nuif * nuj / (nuif + nuj);
-            } else {
-                cmu = nuif;
+        constexpr int B = 3;
+        for (int k0 = 0; k0 < n; k0 += B) {
+            int js[B], ts[B];
+            float z1s[B], z2s[B], pds[B];
+            float4 ks[B], ws[B], ps[B], vs[B];
+            uint8_t fs[B];
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                const long e = ell(r, min(k0 + m, n - 1), kmax);
+                js[m] = D.nidx[e];
+                z1s[m] = ld<float>(D.nkx, e);
+                z2s[m] = ld<float>(D.nky, e);
+                pds[m] = ld<float>(D.nrinv, e);
             }
-            float vart = 0.0f;
-            if (freei) vart = vartsif;
-            else if (D.flags[j] & BS_FLAG_FREE) vart = bs_Wf(ld<float>(D.ndist, e), KF) * wj.y * iwo;
-            const float pvol = wj.x;
-            const float Lx = cf.lx(z1, z2), Ly = cf.ly(z1, z2);
-            const float4 pj4 = __ldg(D.pos4 + j), vj4 = __ldg(D.rec0 + j);
-            const float dxi = f2_diff(pi4.x, pi4.y, pj4.x, pj4.y).x, dyi = f2_diff(pi4.z, pi4.w, pj4.z, pj4.w).x;
-            const float gg = 2.0f * pvol * (dxi * Lx + dyi * Ly) * pd;
-            const float ax = f2_diff(vi4.x, vi4.y, vj4.x, vj4.y).x * gg;
-            const float ay = f2_diff(vi4.z, vi4.w, vj4.z, vj4.w).x * gg;
-            kx.add(ax * (cmu + vart));
-            ky.add(ay * (cmu + vart));
-            if (tj > 2) {
-                const float nutj = kj.z;
-                float mix;
-                if (nutis && wj.z != 0.0f) mix = (nutif + nutj) * 0.5f;
-                else mix = (2.0f * nutif * nutj) / (nutif + nutj);
-                kx.add(ax * mix);
-                ky.add(ay * mix);
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                const int j = js[m];
+                ts[m] = D.tid[j];
+                fs[m] = D.flags[j];
+                ks[m] = __ldg(D.rec1 + j);
+                ws[m] = __ldg(D.rec2 + j);
+                ps[m] = __ldg(D.pos4 + j);
+                vs[m] = __ldg(D.rec0 + j);
             }
-            const float tk = pvol * f2_diff(kj.x, kj.y, ki4.x, ki4.y).x;
-            kx.add(-(tk * Lx * phif * two3f));
-            ky.add(-(tk * Ly * phif * two3f));
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                if (k0 + m >= n) break;
+                const int tj = ts[m];
+                const float z1 = z1s[m], z2 = z2s[m], pd = pds[m];
+                const float4 kj = ks[m], wj = ws[m], pj4 = ps[m], vj4 = vs[m];
+                float cmu;
+                if (tj == BS_TID_FLUID) {   // harmonic mean
+                    const float nuj = kj.w;
+                    cmu = 2.0f * nuif * nuj / (nuif + nuj);
+                } else {
+                    cmu = nuif;
+                }
+                float vart = 0.0f;
+                if (freei) vart = vartsif;
+                else if (fs[m] & BS_FLAG_FREE) vart = bs_Wf(ld<float>(D.ndist, ell(r, k0 + m, kmax)), KF) * wj.y * iwo;
+                const float pvol = wj.x;
+                const float Lx = cf.lx(z1, z2), Ly = cf.ly(z1, z2);
+                const float dxi = f2_diff(pi4.x, pi4.y, pj4.x, pj4.y).x, dyi = f2_diff(pi4.z, pi4.w, pj4.z, pj4.w).x;
+                const float gg = 2.0f * pvol * (dxi * Lx + dyi * Ly) * pd;
+                const float ax = f2_diff(vi4.x, vi4.y, vj4.x, vj4.y).x * gg;
+                const float ay = f2_diff(vi4.z, vi4.w, vj4.z, vj4.w).x * gg;
+                kx.add(ax * (cmu + vart));
+                ky.add(ay * (cmu + vart));
+                if (tj > 2) {
+                    const float nutj = kj.z;
+                    float mix;
+                    if (nutis && wj.z != 0.0f) mix = (nutif + nutj) * 0.5f;
+                    else mix = (2.0f * nutif * nutj) / (nutif + nutj);
+                    kx.add(ax * mix);
+                    ky.add(ay * mix);
+                }
+                const float tk = pvol * f2_diff(kj.x, kj.y, ki4.x, ki4.y).x;
+                kx.add(-(tk * Lx * phif * two3f));
+                ky.add(-(tk * Ly * phif * two3f));
+            }
         }
         sxd = kx.value();
         syd = ky.value();
@@ -807,63 +859,82 @@ __device__ __forceinline__ void assemble_mixed(const Dev& D, const RowCtx& R) {
     float* a32 = D.aval32;
     Kahan32 dia;
     float2 fv = make_float2(0.0f, 0.0f);
-    for (int k = 0; k < n; ++k) {
-        const long e = ell(r, k, kmax);
-        const int j = D.nidx[e];
-        const float z1 = ld<float>(D.nkx, e), z2 = ld<float>(D.nky, e);
-        const float pd = ld<float>(D.nrinv, e);
-        const int tj = D.tid[j];
-        const float4 pj4 = __ldg(D.pos4 + j);
-        const float dxi = f2_diff(pi4.x, pi4.y, pj4.x, pj4.y).x;   // x_i - x_j
-        const float dyi = f2_diff(pi4.z, pi4.w, pj4.z, pj4.w).x;
-        float off = 0.0f;
-        if (ti == BS_TID_FLUID) {
-            const float4 aj4 = __ldg(D.rec2 + j);
-            const float lamp = (freei && tj == BS_TID_FLUID) ? (1.0f + aj4.z * lampf) : 1.0f;
-            const float pvol = aj4.y;
-            const float2 Lx = cf.lx2(z1, z2), Ly = cf.ly2(z1, z2);
-            const float t12 = 2.0f * pvol * (Lx.x * dxi + Ly.x * dyi) * pd;
-            off = -t12;
-            dia.add(t12 * lamp);
-            float2 ax, ay;
-            if (tj == BS_TID_FLUID) {
-                const float aj = aj4.x;
-                const float rho_ij = 2.0f * aj * ai / (aj + ai);
-                const float4 uj = __ldg(D.rec0 + j);
-                ax = f2_mulf(f2_diff(uj.x, uj.y, ui.x, ui.y), rho_ij);
-                ay = f2_mulf(f2_diff(uj.z, uj.w, ui.z, ui.w), rho_ij);
-            } else {
-                const float4 vj = __ldg(D.rec1 + j);
-                ax = f2_mulf(f2_diff(vj.x, vj.y, vi.x, vi.y), bi);
-                ay = f2_mulf(f2_diff(vj.z, vj.w, vi.z, vi.w), bi);
-            }
-            fv = f2_add(fv, f2_mulf(f2_add(f2_mul(ax, Lx), f2_mul(ay, Ly)), pvol));
-        } else if (ti == BS_TID_GHOST) {
-            if (tj <= 2) {
-                const float t12 = 2.0f * __ldg(D.rec2 + j).y * (z1 * dxi + z2 * dyi) * pd;
-                off = -t12;
-                dia.add(t12);
-            }
-        } else if (ti == BS_TID_WALL) {
-            if (tj == BS_TID_FLUID) {
-                const CorrF cj = corr_f(D, j);
-                const float2 Lx = cj.lx2(z1, z2), Ly = cj.ly2(z1, z2);
-                const float t12 = 2.0f * voli * (Lx.x * dxi + Ly.x * dyi) * pd;
-                off = -t12;
-                dia.add(t12);
-                // a_j (u_j/phi_j - vxs_i/phi_i): vxs_i/phi_i is the row's own u/phi
-                const float aj = __ldg(D.rec2 + j).x;
-                const float4 uj = __ldg(D.rec0 + j);
-                const float2 ax = f2_mulf(f2_diff(uj.x, uj.y, ui.x, ui.y), aj);
-                const float2 ay = f2_mulf(f2_diff(uj.z, uj.w, ui.z, ui.w), aj);
-                fv = f2_add(fv, f2_mulf(f2_add(f2_mul(ax, Lx), f2_mul(ay, Ly)), voli));
-            } else {
-                const float t12 = 2.0f * __ldg(D.rec2 + j).y * (z1 * dxi + z2 * dyi) * pd;
-                off = -t12;
-                dia.add(t12);
-            }
+    constexpr int B = 2;   // neighbours loaded at once
+    for (int k0 = 0; k0 < n; k0 += B) {
+        int js[B], ts[B];
+        float z1s[B], z2s[B], pds[B];
+        float4 ps[B], as[B], us[B];
+#pragma unroll
+        for (int m = 0; m < B; ++m) {
+            const long e = ell(r, min(k0 + m, n - 1), kmax);
+            js[m] = D.nidx[e];
+            z1s[m] = ld<float>(D.nkx, e);
+            z2s[m] = ld<float>(D.nky, e);
+            pds[m] = ld<float>(D.nrinv, e);
         }
-        a32[e] = off;   // unscaled, scaled below
+#pragma unroll
+        for (int m = 0; m < B; ++m) {
+            ts[m] = D.tid[js[m]];
+            ps[m] = __ldg(D.pos4 + js[m]);
+            as[m] = __ldg(D.rec2 + js[m]);
+        }
+#pragma unroll
+        for (int m = 0; m < B; ++m)   // u/phi of fluid, vxs of others
+            us[m] = __ldg((ts[m] == BS_TID_FLUID ? D.rec0 : D.rec1) + js[m]);
+#pragma unroll
+        for (int m = 0; m < B; ++m) {
+            if (k0 + m >= n) break;
+            const long e = ell(r, k0 + m, kmax);
+            const int j = js[m], tj = ts[m];
+            const float z1 = z1s[m], z2 = z2s[m], pd = pds[m];
+            const float4 pj4 = ps[m], aj4 = as[m], uj = us[m];
+            const float dxi = f2_diff(pi4.x, pi4.y, pj4.x, pj4.y).x;   // x_i - x_j
+            const float dyi = f2_diff(pi4.z, pi4.w, pj4.z, pj4.w).x;
+            float off = 0.0f;
+            if (ti == BS_TID_FLUID) {
+                const float lamp = (freei && tj == BS_TID_FLUID) ? (1.0f + aj4.z * lampf) : 1.0f;
+                const float pvol = aj4.y;
+                const float2 Lx = cf.lx2(z1, z2), Ly = cf.ly2(z1, z2);
+                const float t12 = 2.0f * pvol * (Lx.x * dxi + Ly.x * dyi) * pd;
+                off = -t12;
+                dia.add(t12 * lamp);
+                float2 ax, ay;
+                if (tj == BS_TID_FLUID) {
+                    const float aj = aj4.x;
+                    const float rho_ij = 2.0f * aj * ai / (aj + ai);
+                    ax = f2_mulf(f2_diff(uj.x, uj.y, ui.x, ui.y), rho_ij);
+                    ay = f2_mulf(f2_diff(uj.z, uj.w, ui.z, ui.w), rho_ij);
+                } else {
+                    ax = f2_mulf(f2_diff(uj.x, uj.y, vi.x, vi.y), bi);
+                    ay = f2_mulf(f2_diff(uj.z, uj.w, vi.z, vi.w), bi);
+                }
+                fv = f2_add(fv, f2_mulf(f2_add(f2_mul(ax, Lx), f2_mul(ay, Ly)), pvol));
+            } else if (ti == BS_TID_GHOST) {
+                if (tj <= 2) {
+                    const float t12 = 2.0f * aj4.y * (z1 * dxi + z2 * dyi) * pd;
+                    off = -t12;
+                    dia.add(t12);
+                }
+            } else if (ti == BS_TID_WALL) {
+                if (tj == BS_TID_FLUID) {
+                    const CorrF cj = corr_f(D, j);
+                    const float2 Lx = cj.lx2(z1, z2), Ly = cj.ly2(z1, z2);
+                    const float t12 = 2.0f * voli * (Lx.x * dxi + Ly.x * dyi) * pd;
+                    off = -t12;
+                    dia.add(t12);
+                    // a_j (u_j/phi_j - vxs_i/phi_i): vxs_i/phi_i is the row's own u/phi
+                    const float aj = aj4.x;
+                    const float2 ax = f2_mulf(f2_diff(uj.x, uj.y, ui.x, ui.y), aj);
+                    const float2 ay = f2_mulf(f2_diff(uj.z, uj.w, ui.z, ui.w), aj);
+                    fv = f2_add(fv, f2_mulf(f2_add(f2_mul(ax, Lx), f2_mul(ay, Ly)), voli));
+                } else {
+                    const float t12 = 2.0f * aj4.y * (z1 * dxi + z2 * dyi) * pd;
+                    off = -t12;
+                    dia.add(t12);
+                }
+            }
+            a32[e] = off;   // unscaled, scaled below
+        }
     }
     double extra = 0.0;
     if (ti == BS_TID_GHOST && n > 0) {
@@ -879,14 +950,22 @@ __device__ __forceinline__ void assemble_mixed(const Dev& D, const RowCtx& R) {
     // double-float split off * (inv hi + inv lo) for the solver's SpMV
     const float2 invd = f2_split(inv);
     double* a = (double*)D.aval;
-    for (int k = 0; k < n; ++k) {
-        const long e = ell(r, k, kmax);
-        const float o = a32[e];
-        const float ph = __fmul_rn(o, invd.x);
-        const float2 v = f2_fast_two_sum(ph, __fmaf_rn(o, invd.y, __fmaf_rn(o, invd.x, -ph)));
-        a32[e] = v.x;
-        D.aval_lo[e] = v.y;
-        a[e] = (double)o * inv;
+    constexpr int BO = 4;
+    for (int k0 = 0; k0 < n; k0 += BO) {
+        float os[BO];
+#pragma unroll
+        for (int m = 0; m < BO; ++m) os[m] = a32[ell(r, min(k0 + m, n - 1), kmax)];
+#pragma unroll
+        for (int m = 0; m < BO; ++m) {
+            if (k0 + m >= n) break;
+            const long e = ell(r, k0 + m, kmax);
+            const float o = os[m];
+            const float ph = __fmul_rn(o, invd.x);
+            const float2 v = f2_fast_two_sum(ph, __fmaf_rn(o, invd.y, __fmaf_rn(o, invd.x, -ph)));
+            a32[e] = v.x;
+            D.aval_lo[e] = v.y;
+            a[e] = (double)o * inv;
+        }
     }
     if (r == P.row0) D.dyn[R.s].asm_split = 1;
 }
@@ -1023,17 +1102,35 @@ __global__ void __launch_bounds__(BS_THREADS) k_compvel(Dev D, int do_vel, int d
                 const CorrF cf = corr_f(D, r);
                 const float rhoif = (float)rhoi;
                 Kahan32 kx, ky;
-                for (int k = 0; k < n; ++k) {
-                    const long e = ell(r, k, kmax);
-                    const int j = D.nidx[e];
-                    const float z1 = ld<float>(D.nkx, e), z2 = ld<float>(D.nky, e);
-                    const float Lx = cf.lx(z1, z2), Ly = cf.ly(z1, z2);
-                    const float4 qj = __ldg(D.rec0 + j);   // (p, rho/phi, m/rho)
-                    float q;
-                    if (D.tid[j] == BS_TID_FLUID) q = qff * qj.z * (qj.x * aif + pif * qj.y) / (aif + qj.y);
-                    else q = qj.z * phi2f * (qj.x + pif) / rhoif;
-                    kx.add(-(q * Lx));
-                    ky.add(-(q * Ly));
+                constexpr int B = 4;
+                for (int k0 = 0; k0 < n; k0 += B) {
+                    int js[B], ts[B];
+                    float z1s[B], z2s[B];
+                    float4 qs[B];
+#pragma unroll
+                    for (int m = 0; m < B; ++m) {
+                        const long e = ell(r, min(k0 + m, n - 1), kmax);
+                        js[m] = D.nidx[e];
+                        z1s[m] = ld<float>(D.nkx, e);
+                        z2s[m] = ld<float>(D.nky, e);
+                    }
+#pragma unroll
+                    for (int m = 0; m < B; ++m) {
+                        qs[m] = __ldg(D.rec0 + js[m]);   // (p, rho/phi, m/rho)
+                        ts[m] = D.tid[js[m]];
+                    }
+#pragma unroll
+                    for (int m = 0; m < B; ++m) {
+                        if (k0 + m >= n) break;
+                        const float z1 = z1s[m], z2 = z2s[m];
+                        const float Lx = cf.lx(z1, z2), Ly = cf.ly(z1, z2);
+                        const float4 qj = qs[m];
+                        float q;
+                        if (ts[m] == BS_TID_FLUID) q = qff * qj.z * (qj.x * aif + pif * qj.y) / (aif + qj.y);
+                        else q = qj.z * phi2f * (qj.x + pif) / rhoif;
+                        kx.add(-(q * Lx));
+                        ky.add(-(q * Ly));
+                    }
                 }
                 axd = kx.value();
                 ayd = ky.value();
@@ -1257,35 +1354,53 @@ __global__ void __launch_bounds__(BS_THREADS) k_scalar(Dev D, int substep, const
         const float4 pi4 = D.pos4[r];
         const KerF KF = ker_f(P);
         float cdf = 0.0f;
-        for (int k = 0; k < n; ++k) {
-            const long e = ell(r, k, kmax);
-            const int j = D.nidx[e];
-            if (D.tid[j] != BS_TID_FLUID) continue;
-            const float4 sj = __ldg(D.rec1 + j);   // (Dt, con, phi, flags)
-            const int bits = (int)sj.w;
-            const float pj = sj.z;
-            const float dm = ld<float>(D.ndist, e);
-            const float4 pj4 = __ldg(D.pos4 + j);
-            const float dx = f2_diff(pi4.x, pi4.y, pj4.x, pj4.y).x, dy = f2_diff(pi4.z, pi4.w, pj4.z, pj4.w).x;
-            float t1x;
-            if (psmall && (bits & 1)) {
-                const float4 dj = __ldg(D.rec0 + j);
-                const float Dxx = P0 + dj.x, Dxy = P1 + dj.y;
-                const float Dyx = P2 + dj.z, Dyy = P3 + dj.w;
-                const float ph = 0.5f / dm;
-                const float A = Dxx * dx * ph + Dxy * dy * ph, B = Dyx * dx * ph + Dyy * dy * ph;
-                t1x = 1.0f / (A * A + B * B);
-                t1x = (t1x <= capf) ? t1x : capf;
-            } else {
-                const float Dj = sj.x;
-                if (nsmall && (bits & 2)) t1x = (Dtf + Dj) * 0.5f;
-                else t1x = 2.0f * Dtf * Dj / (Dtf + Dj);
+        constexpr int B = 3;
+        for (int k0 = 0; k0 < n; k0 += B) {
+            int js[B], ts[B];
+            float dms[B], pds[B];
+            float4 ss[B], ps[B];
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                const long e = ell(r, min(k0 + m, n - 1), kmax);
+                js[m] = D.nidx[e];
+                dms[m] = ld<float>(D.ndist, e);
+                pds[m] = ld<float>(D.nrinv, e);
             }
-            const float t3 = ovf * (phif + pj) / (phif * pj);
-            const float F = bs_Ff(dm, KF);
-            const float pd = ld<float>(D.nrinv, e);
-            const float dc = cof - sj.y;
-            cdf += t1x * t3 * dc * (dx * (F * dx) + dy * (F * dy)) * pd;
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                ts[m] = D.tid[js[m]];
+                ss[m] = __ldg(D.rec1 + js[m]);   // (Dt, con, phi, flags)
+                ps[m] = __ldg(D.pos4 + js[m]);
+            }
+#pragma unroll
+            for (int m = 0; m < B; ++m) {
+                if (k0 + m >= n) break;
+                if (ts[m] != BS_TID_FLUID) continue;
+                const float4 sj = ss[m], pj4 = ps[m];
+                const int bits = (int)sj.w;
+                const float pj = sj.z;
+                const float dm = dms[m];
+                const float dx = f2_diff(pi4.x, pi4.y, pj4.x, pj4.y).x, dy = f2_diff(pi4.z, pi4.w, pj4.z, pj4.w).x;
+                float t1x;
+                if (psmall && (bits & 1)) {
+                    const float4 dj = __ldg(D.rec0 + js[m]);
+                    const float Dxx = P0 + dj.x, Dxy = P1 + dj.y;
+                    const float Dyx = P2 + dj.z, Dyy = P3 + dj.w;
+                    const float ph = 0.5f / dm;
+                    const float A = Dxx * dx * ph + Dxy * dy * ph, B = Dyx * dx * ph + Dyy * dy * ph;
+                    t1x = 1.0f / (A * A + B * B);
+                    t1x = (t1x <= capf) ? t1x : capf;
+                } else {
+                    const float Dj = sj.x;
+                    if (nsmall && (bits & 2)) t1x = (Dtf + Dj) * 0.5f;
+                    else t1x = 2.0f * Dtf * Dj / (Dtf + Dj);
+                }
+                const float t3 = ovf * (phif + pj) / (phif * pj);
+                const float F = bs_Ff(dm, KF);
+                const float pd = pds[m];
+                const float dc = cof - sj.y;
+                cdf += t1x * t3 * dc * (dx * (F * dx) + dy * (F * dy)) * pd;
+            }
         }
         cd = cdf;
     }
