@@ -213,6 +213,11 @@ bs::Launch launch_of(bs_ctx* c) {
     L.mgchip_smem = c->mgchip_smem;
     L.mgsub_cs = c->mgsub_cs;
     L.sweep_tpb = c->sweep_tpb;
+    // A small scene's sweeps in blocks small enough for two on each SM: its FP64
+    // pair arithmetic is bound by each SM's pipe (13,681 rows of 30 neighbours on
+    // 54 SMs in blocks of 256, on all in blocks of 32: search 477 and 333 us, int_vel
+    // 228 and 171; 15 k rows in mixed precision take the same either way).
+    while (L.sweep_tpb > 32 && (long)c->nblk_total * (BS_THREADS / L.sweep_tpb) < 2L * c->sm_count) L.sweep_tpb /= 2;
     L.mg0_tpb = c->mg0_tpb;
     L.exact = &c->mgexact;
     return L;

@@ -609,7 +609,7 @@ struct Launch {
     int mgsub_level, mgsub_cs;     // first level of the clustered subtree (0: per-level launches), CTAs per cluster
     int mgtail;                    // level whose visits run on chip, everything below included (0: none)
     int mgchip_cs, mgchip_smem;    // ... blocks per cluster and bytes of shared memory per block
-    int sweep_tpb;                 // threads per block of the neighbour sweeps (64, 128 or 256)
+    int sweep_tpb;                 // threads per block of the neighbour sweeps (32, 64, 128 or 256)
     int mg0_tpb;                   // threads per block of the particle-level multigrid kernels
     const MgExact* exact;          // the scenes' exactly solved levels (when D.mg.exact)
 };
