@@ -361,54 +361,81 @@ __global__ void __launch_bounds__(BS_THREADS, 4) k_search(Dev D, int do_search, 
                 const float t2f = t2c * (1.0f + 1e-5f);
                 float4 pi4 = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (sizeof(T) == 4) pi4 = D.pos4[r];
-                for (int k = 0; k < 4; ++k) {
-                    const int q = (ordp >> (2 * k)) & 3;
-                    const int di = di0 + (q & 1), dj = dj0 + (q >> 1);
-                    const int cq = c + dj * P.celly + di;
-                    float ox, oy;
-                    cell_offset(cwf, dj, di, ox, oy);
-                    const int g1 = D.gcell_end[cq];
-                    for (int g0 = D.gcell_start[cq]; g0 < g1; g0 += NG) {
-                        // FP32 prefilter (as in the neighbour scan): a grain
-                        // rejected here is outside 2h in FP64 as well
-                        // (the arrays run NG past the last grain, as the rows')
-                        const float *const fx0 = D.gxr + g0, *const fy0 = D.gyr + g0;
-                        float xs[NG], ys[NG];
+                // Up to four chunks of 32 grains (the four cells of a usual
+                // scene) are tested into a mask each before the first accepted
+                // grain is summed: a warp then takes as many rounds as its
+                // lane with the most grains, not the most of every batch (FP64: 333
+                // and 194 us at 13,681 rows among grains, 604 and 483 at 187 k; mixed:
+                // 103 and 99 at 187 k, 438 and 445 at 1.04 M).
+                int k = -1, g = 0, g1 = 0;
+                float ox = 0.0f, oy = 0.0f;
+                while (k < 4) {
+                    unsigned mask[4];
+                    int from[4];
 #pragma unroll
-                        for (int m = 0; m < NG; ++m) {
-                            xs[m] = __ldg(fx0 + m);
-                            ys[m] = __ldg(fy0 + m);
+                    for (int u = 0; u < 4; ++u) {
+                        mask[u] = 0;
+                        while (g >= g1 && ++k < 4) {
+                            const int q = (ordp >> (2 * k)) & 3;
+                            const int di = di0 + (q & 1), dj = dj0 + (q >> 1);
+                            const int cq = c + dj * P.celly + di;
+                            cell_offset(cwf, dj, di, ox, oy);
+                            g = D.gcell_start[cq];
+                            g1 = D.gcell_end[cq];
                         }
-                        unsigned in = 0;
+                        from[u] = g;
+                        if (k >= 4) continue;
+#pragma unroll 1
+                        for (int b = 0; b < 32 && g + b < g1; b += NG) {
+                            // FP32 prefilter (as in the neighbour scan): a grain
+                            // rejected here is outside 2h in FP64 as well
+                            // (the arrays run NG past the last grain, as the rows')
+                            const float *const gx = D.gxr + g + b, *const gy = D.gyr + g + b;
+                            float xs[NG], ys[NG];
 #pragma unroll
-                        for (int m = 0; m < NG; ++m) {
-                            const float fx = (xs[m] + ox) - rel.x, fy = (ys[m] + oy) - rel.y;
-                            if (!(fx * fx + fy * fy > t2f)) in |= 1u << m;
-                        }
-                        in &= ((1u << BS_CAND) - 1) >> max(NG - (g1 - g0), 0);
-                        for (; in; in &= in - 1) {
-                            const int g = g0 + __ffs(in) - 1;
-                            if (sizeof(T) == 4) {
-                                // mixed: FP32 (W(2h) = 0: the cut needs no exact
-                                // test), the offset from the double-float positions
-                                const float4 g4 = __ldg(D.gpos4 + g);
-                                const float ex = f2_diff(pi4.x, pi4.y, g4.x, g4.y).x;
-                                const float ey = f2_diff(pi4.z, pi4.w, g4.z, g4.w).x;
-                                const float s2 = ex * ex + ey * ey;
-                                if (s2 < t2c) {
-                                    float rad = 0.0f;   // grains may coincide with pore particles
-                                    if (s2 > 0.0f) {
-                                        float ir = rsqrtf(s2);
-                                        ir = ir * (1.5f - 0.5f * s2 * ir * ir);
-                                        rad = s2 * ir;
-                                    }
-                                    sff.add(wsf * bs_Wf(rad, KF) * (float)D.gv[g]);
-                                }
-                            } else {
-                                const double dx = xi - D.gx[g], dy = yi - D.gy[g];
-                                const double rad = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-                                if (rad < P.twoh) sf = sf + wsolid * bs_W(rad, P) * D.gv[g];
+                            for (int m = 0; m < NG; ++m) {
+                                xs[m] = __ldg(gx + m);
+                                ys[m] = __ldg(gy + m);
                             }
+                            unsigned in = 0;
+#pragma unroll
+                            for (int m = 0; m < NG; ++m) {
+                                const float fx = (xs[m] + ox) - rel.x, fy = (ys[m] + oy) - rel.y;
+                                if (!(fx * fx + fy * fy > t2f)) in |= 1u << m;
+                            }
+                            in &= ((1u << BS_CAND) - 1) >> max(NG - (g1 - g - b), 0);
+                            mask[u] |= in << b;
+                        }
+                        g += 32;
+                    }
+#pragma unroll 1
+                    while (mask[0] | mask[1] | mask[2] | mask[3]) {
+                        const int u = mask[0] ? 0 : mask[1] ? 1 : mask[2] ? 2 : 3;
+                        const unsigned in = u == 0 ? mask[0] : u == 1 ? mask[1] : u == 2 ? mask[2] : mask[3];
+                        const int g = (u == 0 ? from[0] : u == 1 ? from[1] : u == 2 ? from[2] : from[3]) + __ffs(in) - 1;
+#pragma unroll
+                        for (int v = 0; v < 4; ++v)
+                            if (v == u) mask[v] &= mask[v] - 1;
+                        if (sizeof(T) == 4) {
+                            // mixed: FP32 (W(2h) = 0: the cut needs no exact
+                            // test), the offset from the double-float positions
+                            const float4 g4 = __ldg(D.gpos4 + g);
+                            const float ex = f2_diff(pi4.x, pi4.y, g4.x, g4.y).x;
+                            const float ey = f2_diff(pi4.z, pi4.w, g4.z, g4.w).x;
+                            const float s2 = ex * ex + ey * ey;
+                            if (s2 < t2c) {
+                                float rad = 0.0f;   // grains may coincide with pore particles
+                                if (s2 > 0.0f) {
+                                    float ir = rsqrtf(s2);
+                                    ir = ir * (1.5f - 0.5f * s2 * ir * ir);
+                                    rad = s2 * ir;
+                                }
+                                sff.add(wsf * bs_Wf(rad, KF) * (float)D.gv[g]);
+                            }
+                        } else {
+                            const double dx = xi - D.gx[g], dy = yi - D.gy[g];
+                            const double rad = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+                            if (rad < P.twoh) sf = sf + wsolid * bs_W(rad, P) * D.gv[g];
                         }
                     }
                 }
