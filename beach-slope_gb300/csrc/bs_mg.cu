@@ -79,6 +79,7 @@ __global__ void k_mg_gal0(Dev D) {
     const int r0 = D.cell_start[c], r1 = D.cell_end[c];
     const T* A = (const T*)(sizeof(T) == 8 ? D.aval : (void*)D.aval32);
     const uint8_t* sub = D.mg.sub;
+    constexpr int B = 4;   // neighbours loaded at once
     T mine0 = 0, mine1 = 0;
     for (int base = r0; base < r1; base += 32) {
         const int r = base + lane;
@@ -91,21 +92,34 @@ __global__ void k_mg_gal0(Dev D) {
             const int si = sb & 1, sj = sb >> 1;
             acc[4] += (T)D.adiag[r];
             const int n = D.ncount[r];
-            for (int k = 0; k < n; ++k) {
-                const long e = ell(r, k, D.kmax);
-                const int col = D.nidx[e];
-                const int d = D.cell[col] - c;
-                const int u = d + celly + 1;   // in [0, 2 celly + 2] for the 3x3 neighbour cells
-                const int dj = (u >= 2 * celly) ? 1 : ((u >= celly) ? 0 : -1);
-                const int di = d - dj * celly;
-                const int s2 = sub[col];
-                const int dI = min(max(2 * di + (s2 & 1) - si, -1), 1);
-                const int dJ = min(max(2 * dj + (s2 >> 1) - sj, -1), 1);
-                const int q = (dJ + 1) * 3 + (dI + 1);
-                const T v = A[e];
+            for (int k0 = 0; k0 < n; k0 += B) {
+                int cols[B], cells[B], subs[B];
+                T vs[B];
 #pragma unroll
-                for (int t = 0; t < 9; ++t)
-                    if (t == q) acc[t] += v;
+                for (int m = 0; m < B; ++m) {
+                    const long e = ell(r, min(k0 + m, n - 1), D.kmax);
+                    cols[m] = D.nidx[e];
+                    vs[m] = A[e];
+                }
+#pragma unroll
+                for (int m = 0; m < B; ++m) {
+                    cells[m] = D.cell[cols[m]];
+                    subs[m] = sub[cols[m]];
+                }
+#pragma unroll
+                for (int m = 0; m < B; ++m) {
+                    const int d = cells[m] - c;
+                    const int u = d + celly + 1;   // in [0, 2 celly + 2] for the 3x3 neighbour cells
+                    const int dj = (u >= 2 * celly) ? 1 : ((u >= celly) ? 0 : -1);
+                    const int di = d - dj * celly;
+                    const int s2 = subs[m];
+                    const int dI = min(max(2 * di + (s2 & 1) - si, -1), 1);
+                    const int dJ = min(max(2 * dj + (s2 >> 1) - sj, -1), 1);
+                    const int q = (dJ + 1) * 3 + (dI + 1);
+#pragma unroll
+                    for (int t = 0; t < 9; ++t)
+                        if (t == q && k0 + m < n) acc[t] += vs[m];
+                }
             }
         }
 #pragma unroll
