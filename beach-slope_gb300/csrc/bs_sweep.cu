@@ -1498,8 +1498,10 @@ __device__ __forceinline__ void pow7(double x, double& h, double& e) {
 // the root 27: FP32's root, then two Newton steps, the second with the residual
 // x - y^7 to twice the precision (before the last rounding y is good to 1e-18, the
 // power to 1e-31: no less than pow's).  Outside FP32's range and for other
-// exponents, pow.  1.04 M rows, before and now: the hydrostatic density 217 and
-// %s us, the equation of state with its inverse 231 and %s.
+// exponents, pow.  Largest errors against extended precision at densities of 0.95
+// to 2 of the reference: root 2.2e-16 both ways, power 2.5e-16 with pow and 2.0e-16.
+// 1.04 M rows, before and now: the hydrostatic density 217 and 84 us, the equation
+// of state with its inverse 231 and 93.
 __device__ __forceinline__ double tait_pow(double x, double gam) {
     if (gam != 7.0) return pow(x, gam);
     double h, e;
