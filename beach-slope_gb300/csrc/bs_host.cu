@@ -2139,10 +2139,16 @@ static int krylov_csr(int solver, int32_t n, const int32_t* row_ptr, const int32
     CK(cudaMemcpy(D.aval, aval.data(), sizeof(double) * E, cudaMemcpyHostToDevice));
     ctx->assembled = true;
     D.fg_df = 0;
+    // Columns and iterations per graph launch and read of the converged count (4 us of
+    // a column's or an iteration's time): FGMRES 10.2 -> 7.8 ms at 60,025 rows,
+    // BiCGStab 4.43 -> 4.13 at 2,500; what a chunk runs past the end are empty
+    // launches, five per iteration of BiCGStab: 100 us, more than the few iterations
+    // of a system below 1,024 rows gain.
+    const int chunk = solver == BS_SOLVER_FGMRES || n >= 1024 ? 8 : 1;
     if (solver == BS_SOLVER_FGMRES)
-        bs::solve_fgmres(D, launch_of(ctx), maxit, 1, 0, BS_PREC_FP64, ctx->d_nconv, ctx->h_pinned, ctx->evsync);
+        bs::solve_fgmres(D, launch_of(ctx), maxit, chunk, 0, BS_PREC_FP64, ctx->d_nconv, ctx->h_pinned, ctx->evsync);
     else
-        bs::solve_fp64(D, launch_of(ctx), maxit, 1, 0, BS_PREC_FP64, ctx->d_nconv, ctx->h_pinned, ctx->evsync);
+        bs::solve_fp64(D, launch_of(ctx), maxit, chunk, 0, BS_PREC_FP64, ctx->d_nconv, ctx->h_pinned, ctx->evsync);
     rc = bs_sync(ctx);
     if (!rc) {
         CK(cudaMemcpy(x, D.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
