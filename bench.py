@@ -163,7 +163,7 @@ TIMED_KERNELS = ("search_effpor", "bicg_it1_spmv", "bicg_it2_spmv", "mg_l0_down"
 # launch (ncu dram__bytes_read.sum + dram__bytes_write.sum on the 0.18 M-particle beach, mixed);
 # the traffic grows with the nonzeros and rows, so the ratio scales it to the
 # bench's workload.  k_it2_64 has k_it1_64's access pattern.  fg_arnoldi_spmv:
-# every launch of seven solves of the double-float form (k_fg_arn1<1>) the
+# every launch of seven solves of the double-float form (k_fg_arn1_df) the
 # mixed bench times.
 TRAFFIC_RATIO = {"search_effpor": 0.46, "bicg_it1_spmv": 0.99, "bicg_it2_spmv": 0.99,
                  "mg_l0_down": 0.99, "mg_l0_up": 0.93, "fg_arnoldi_spmv": 0.90, "fg_project": 0.97}
