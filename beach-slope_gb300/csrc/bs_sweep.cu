@@ -1484,46 +1484,10 @@ namespace bs {
 // ------------------------------------------------------------------ WCSPH
 // wcsph.f90, a module the reference ships but never calls.
 
-// x^7 as a rounded value and its remainder: products with their rounding errors
-// (TwoProduct by fused multiply-add, Ogita, Rump and Oishi 2005).
-__device__ __forceinline__ void pow7(double x, double& h, double& e) {
-    const double x2 = __dmul_rn(x, x), e2 = __fma_rn(x, x, -x2);
-    const double x4 = __dmul_rn(x2, x2), e4 = __fma_rn(2.0 * x2, e2, __fma_rn(x2, x2, -x4));
-    const double x6 = __dmul_rn(x4, x2), e6 = __fma_rn(x4, e2, __fma_rn(x2, e4, __fma_rn(x4, x2, -x6)));
-    h = __dmul_rn(x6, x);
-    e = __fma_rn(x, e6, __fma_rn(x6, x, -h));
-}
-// Tait's power x^gam and root x^(1/gam).  pow is 120 FP64 instructions, and one
-// holds the SM's pipe for 16 cycles; for water's exponent 7 the power is 14 and
-// the root 27: FP32's root, then two Newton steps, the second with the residual
-// x - y^7 to twice the precision (before the last rounding y is good to 1e-18, the
-// power to 1e-31: no less than pow's).  Outside FP32's range and for other
-// exponents, pow.  Largest errors against extended precision at densities of 0.95
-// to 2 of the reference: root 2.2e-16 both ways, power 2.5e-16 with pow and 2.0e-16.
-// 1.04 M rows, before and now: the hydrostatic density 217 and 84 us, the equation
-// of state with its inverse 231 and 93.
-__device__ __forceinline__ double tait_pow(double x, double gam) {
-    if (gam != 7.0) return pow(x, gam);
-    double h, e;
-    pow7(x, h, e);
-    return isfinite(h) ? h + e : h;
-}
-__device__ __forceinline__ double tait_root(double x, double gam) {
-    const int hi = __double2hiint(x);
-    if (gam != 7.0 || hi < (1023 - 100) << 20 || hi >= (1023 + 100) << 20) return pow(x, 1.0 / gam);
-    double y = (double)exp2f(log2f((float)x) * (1.0f / 7.0f));
-    const double y2 = y * y, y6 = y2 * y2 * y2;
-    const double r = (double)__fdividef(1.0f, 7.0f * (float)y6);   // 1 / (7 y^6)
-    y = __fma_rn(__fma_rn(-y6, y, x), r, y);
-    double h, e;
-    pow7(y, h, e);
-    return __fma_rn((x - h) - e, r, y);
-}
-
 // hydrostatic Tait density at height y (the term2 expression, wcsph.f90:78-82)
 __device__ __forceinline__ double wc_hyd(const ScenePar& P, double y) {
     const double rho = P.rho, co = P.wc_c0, gam = P.wc_gamma;
-    return rho * tait_root(((((P.wc_ysurf - y) * rho) * fabs(P.g)) * gam) / (rho * (co * co)) + 1.0, gam);
+    return rho * pow(((((P.wc_ysurf - y) * rho) * fabs(P.g)) * gam) / (rho * (co * co)) + 1.0, 1.0 / gam);
 }
 
 // per-row hydrostatic density (one pow per particle, not per pair)
@@ -1623,14 +1587,14 @@ __global__ void k_wc_rows(Dev D, int mode) {
     const bool fluid = D.tid[r] > 2;
     if ((mode & 1) && fluid) d = D.tden[r];
     if ((mode & 2) && fluid) {
-        double p = (rho * (co * co)) * (tait_pow(d / rho, gam) - 1) / gam;
+        double p = (rho * (co * co)) * (pow(d / rho, gam) - 1) / gam;
         if (p < 0.0) {
             p = 0.0;
             d = rho;
         }
         D.p[r] = p;
     }
-    if (mode & 4) d = rho * tait_root((D.p[r] * gam / (rho * (co * co))) + 1, gam);
+    if (mode & 4) d = rho * pow((D.p[r] * gam / (rho * (co * co))) + 1, 1 / gam);
     if (d != D.rho[r]) {
         D.rho[r] = d;
         D.vol[r] = D.mass[r] / d;
