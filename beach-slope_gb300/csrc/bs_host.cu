@@ -9,6 +9,8 @@
 #include <cstdio>
 #include <cstddef>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -1075,6 +1077,14 @@ int bs_download_wait(bs_ctx* ctx, int32_t s, bs_state* o) {
     return 0;
 }
 
+// The live allocations of bs_host_alloc (start -> bytes): memory that a kernel may
+// write from end to end.  Other page-locked memory takes the copies: the runtime
+// tells of an address that it is registered, not how far the registration
+// reaches, nor whether it is read-only, and a store beyond it is a GPU fault
+// where a copy returns an error.
+static std::mutex g_host_mu;
+static std::map<uintptr_t, size_t>& g_host_ranges = *new std::map<uintptr_t, size_t>;   // (never destroyed: arrays freed at exit)
+
 int bs_host_alloc(size_t bytes, void** p) {
     if (!p) return BS_E_ARG;
     *p = nullptr;
@@ -1083,9 +1093,18 @@ int bs_host_alloc(size_t bytes, void** p) {
         *p = nullptr;
         return BS_E_NOMEM;
     }
+    try {
+        std::lock_guard<std::mutex> lk(g_host_mu);
+        g_host_ranges[(uintptr_t)*p] = bytes ? bytes : 1;
+    } catch (...) {   // (no room for the entry: not known, so it takes the copies)
+    }
     return 0;
 }
 int bs_host_free(void* p) {
+    if (p) {
+        std::lock_guard<std::mutex> lk(g_host_mu);
+        g_host_ranges.erase((uintptr_t)p);
+    }
     if (p && cudaFreeHost(p) != cudaSuccess) {
         cudaGetLastError();
         return BS_E_CUDA;
@@ -1093,10 +1112,19 @@ int bs_host_free(void* p) {
     return 0;
 }
 
-// The address of page-locked host memory on the device, if p is such memory
-// (bs_host_alloc, cudaMallocHost, mapped registrations) and aligned to `align`.
-static void* pinned_on_device(void* p, size_t align) {
+// The address on the device of `bytes` bytes at p, if they lie in one allocation
+// of bs_host_alloc that is still there (a caller may have freed it by the
+// runtime's own call) and p is aligned to `align`.
+static void* pinned_on_device(void* p, size_t bytes, size_t align) {
     if ((uintptr_t)p % align) return nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_host_mu);
+        auto it = g_host_ranges.upper_bound((uintptr_t)p);
+        if (it == g_host_ranges.begin()) return nullptr;
+        --it;
+        const size_t at = (uintptr_t)p - it->first;
+        if (at > it->second || bytes > it->second - at) return nullptr;
+    }
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
@@ -1105,14 +1133,14 @@ static void* pinned_on_device(void* p, size_t align) {
     return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
-// bs_download into page-locked buffers by one kernel that writes them over the
-// host link; 1: not this way (pageable buffers).  A copy per field and two
+// bs_download into bs_host_alloc's buffers by one kernel that writes them over the
+// host link; 1: not this way (other buffers).  A copy per field and two
 // synchronous copies took 104 us at 5 k rows and 545 at 712 k, through Python;
 // this way 40 and 400.
 static int download_pinned(bs_ctx* ctx, int32_t s, bs_state* o) {
     const ScenePar& P = ctx->hpar[s];
-    const int rows = std::min((int)o->n, P.cap);
-    if (rows <= 0 || !ctx->h_dyn) return 1;
+    const size_t rows = std::max(0, std::min((int)o->n, P.cap));   // that the kernel may write of each buffer
+    if (rows == 0 || !ctx->h_dyn) return 1;
     Dev& D = ctx->D;
     double* outs[BS_SNAP_MAXF] = {o->x, o->y, o->vx, o->vy, o->p, o->mass, o->rho, o->oden, o->ovol, o->con,
                                   o->xs, o->ys, o->vxs, o->vys, o->porosity, o->resx, o->resy, o->nut, o->tke,
@@ -1124,22 +1152,22 @@ static int download_pinned(bs_ctx* ctx, int32_t s, bs_state* o) {
     for (int f = 0; f < BS_SNAP_MAXF; ++f) {
         if (!outs[f]) continue;
         a.src[a.nf] = srcs[f];
-        if (!(a.dst[a.nf] = (double*)pinned_on_device(outs[f], sizeof(double)))) return 1;
+        if (!(a.dst[a.nf] = (double*)pinned_on_device(outs[f], rows * sizeof(double), sizeof(double)))) return 1;
         a.nf++;
     }
     int* cell = nullptr;
     double* coff = nullptr;
-    if (o->tid && !(a.tid_dst = (int*)pinned_on_device(o->tid, sizeof(int)))) return 1;
-    if (o->pid && !(a.pid_dst = (int*)pinned_on_device(o->pid, sizeof(int)))) return 1;
-    if (o->flags && !(a.flags_dst = (uint8_t*)pinned_on_device(o->flags, 1))) return 1;
-    if (o->cell && !(cell = (int*)pinned_on_device(o->cell, sizeof(int)))) return 1;
-    if (o->coff && !(coff = (double*)pinned_on_device(o->coff, sizeof(double)))) return 1;
+    if (o->tid && !(a.tid_dst = (int*)pinned_on_device(o->tid, rows * sizeof(int), sizeof(int)))) return 1;
+    if (o->pid && !(a.pid_dst = (int*)pinned_on_device(o->pid, rows * sizeof(int), sizeof(int)))) return 1;
+    if (o->flags && !(a.flags_dst = (uint8_t*)pinned_on_device(o->flags, rows, 1))) return 1;
+    if (o->cell && !(cell = (int*)pinned_on_device(o->cell, rows * sizeof(int), sizeof(int)))) return 1;
+    if (o->coff && !(coff = (double*)pinned_on_device(o->coff, 4 * rows * sizeof(double), sizeof(double)))) return 1;
     if (o->tid) a.tid = D.tid;
     if (o->pid) a.pid = D.pid;
     if (o->flags) a.flags = D.flags;
     a.row0 = P.row0;
     a.n = o->n;
-    bs::read_back(D, launch_of(ctx), a, s, rows, ctx->h_dyn, P.cell0, cell, coff);
+    bs::read_back(D, launch_of(ctx), a, s, (int)rows, ctx->h_dyn, P.cell0, cell, coff);
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaGetLastError());
     const int n = ctx->h_dyn->n;

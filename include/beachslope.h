@@ -242,7 +242,9 @@ int bs_destroy(struct bs_ctx* ctx);
 int bs_upload(struct bs_ctx* ctx, int32_t scene, const bs_state* st, const bs_grains* gr);
 /* Page-locked host memory for the arrays of bs_upload / bs_download
  * (cudaMallocHost): copies from and to it run at the host link's full rate
- * and overlap.  Any host memory works with both calls; this is the fast kind. */
+ * and overlap.  Any host memory works with both calls; this is the fast kind:
+ * bs_download writes buffers that lie whole in such allocations by one kernel,
+ * all others (other page-locked memory too) by a copy per field. */
 int bs_host_alloc(size_t bytes, void** p);
 int bs_host_free(void* p);
 int bs_download(struct bs_ctx* ctx, int32_t scene, bs_state* st);
