@@ -27,6 +27,11 @@
 //    computed after the last iteration.  The flag is read back to the host
 //    every BS_STATIC_CHUNK iterations (the call waits for its stream there),
 //    so the call cannot run on a stream that is being captured.
+//  * The iterations are one cooperative launch, which starts when all of its
+//    blocks (one per 256 rows, up to 204 KB of shared memory each) fit on the
+//    device at once: beside other streams' kernels it waits for theirs to end.
+//    Where such a launch is refused (a partition of the device, a green context)
+//    the phases of an iteration are launches of their own.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -90,9 +95,6 @@ __host__ __device__ inline Scr carve(double* base) {
 // rows: 6 us).  Every sum runs in the order of the launch-per-phase form (256-row
 // blocks, then the blocks by 256 threads), with the products fused alike: the
 // iterates are the same.
-//
-// With fewer resident blocks than row blocks (a device shared out) a block takes
-// several in turn, its vectors in memory.
 struct Grid {
     unsigned* count;    // arrivals, counted up over the launch
     unsigned* broken;   // 1: a wait ran out (the launch gives up)
@@ -149,7 +151,6 @@ __device__ __forceinline__ bool sum2(double (&q)[2], double* buf /*[16 * SUM_LD]
     return true;
 }
 
-template <bool ONE>
 __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const double* b, double* x, double* base, int nblk,
                                                              double tol, int maxit, int chunk, int first, int cap) {
     constexpr int NT = BS_STATIC_THREADS;
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const doubl
     double* const sval = (double*)rows_smem;
     int* const scol = (int*)(sval + cap);
     const int t = threadIdx.x;
-    // the block's first rows of the matrix into shared memory (if they fit)
+    // the block's rows of the matrix into shared memory (if they fit)
     const int i0 = blockIdx.x * NT;
     const int nr = min(NT, A.n - i0);
     for (int k = t; k <= nr; k += NT) rp[k] = A.rp[i0 + k];
@@ -175,12 +176,13 @@ __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const doubl
     Grid G{(unsigned*)(S.sc + 24), (unsigned*)(S.sc + 25), 0};
     if (t < 16) sc[t] = S.sc[t];
     __syncthreads();
-    // (A u)_i, i = vb * NT + t; twelve gathers in flight, the sum in entry order
-    auto row = [&](int vb, const double* u) {
+    const int i = i0 + t;   // this thread's row
+    const bool in = i < A.n;
+    // (A u)_i; twelve gathers in flight, the sum in entry order
+    auto row = [&](const double* u) {
         constexpr int B = 12;
         double acc = 0.0;
-        const int i = vb * NT + t;
-        if (held && (ONE || vb == (int)blockIdx.x)) {
+        if (held) {
             const int end = rp[t + 1] - e0;
             for (int e = rp[t] - e0; e < end; e += B) {
                 double ue[B];
@@ -195,12 +197,11 @@ __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const doubl
         }
         return acc;
     };
-    // the sums of q[] over a row block: partials of phase k's set (two sets: a block may be one barrier ahead)
+    // the block's sums of q[]: partials of phase k's set (two sets: a block may be one barrier ahead)
     int phase = 0;
-    auto partial = [&](int vb, double (&q)[2]) {
-        if (!ONE) __syncthreads();   // sh[0] is read of the row block before
+    auto partial = [&](double (&q)[2]) {
         if (sum2(q, sh[0]) && t == 0) {
-            double* p = S.part + ((long)(phase & 1) * BS_STATIC_MAX_BLOCKS + vb) * BS_STATIC_NPART;
+            double* p = S.part + ((long)(phase & 1) * BS_STATIC_MAX_BLOCKS + blockIdx.x) * BS_STATIC_NPART;
             p[0] = q[0];
             p[1] = q[1];
         }
@@ -218,38 +219,27 @@ __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const doubl
         ++phase;
         return true;
     };
-    double r = 0.0, rh = 0.0, p = 0.0, v = 0.0, s = 0.0, w = 0.0, xi = 0.0;   // ONE: this thread's row
-    const int ir = i0 + t;
-    const bool in1 = ir < A.n;
-    if (ONE && in1) {
-        xi = x[ir];
+    double r = 0.0, rh = 0.0, p = 0.0, v = 0.0, s = 0.0, w = 0.0, xi = 0.0;
+    if (in) {
+        xi = x[i];
         if (!first) {
-            r = S.r[ir];
-            rh = S.rh[ir];
-            p = S.p[ir];
-            v = S.v[ir];
+            r = S.r[i];
+            rh = S.rh[i];
+            p = S.p[i];
+            v = S.v[i];
         }
     }
-#define FOR_ROWS                                                    \
-    for (int vb = blockIdx.x; vb < nblk; vb += gridDim.x)           \
-        for (int i = vb * NT + t, in = i < A.n, go = 1; go; go = 0)
     double a[2];
     if (first) {
-        FOR_ROWS {
-            double q[2] = {0.0, 0.0};
-            if (in) {
-                const double bi = b[i];
-                const double ri = bi - row(vb, x);
-                S.r[i] = ri;
-                S.rh[i] = ri;
-                S.p[i] = 0.0;
-                S.v[i] = 0.0;
-                if (ONE) r = rh = ri;
-                q[0] = __dmul_rn(bi, bi);
-                q[1] = __dmul_rn(ri, ri);
-            }
-            partial(vb, q);
+        double q[2] = {0.0, 0.0};
+        if (in) {
+            const double bi = b[i];
+            r = rh = bi - row(x);
+            S.rh[i] = rh;
+            q[0] = __dmul_rn(bi, bi);
+            q[1] = __dmul_rn(r, r);
         }
+        partial(q);
         if (!total(a)) return;
         if (t == 0) {
             sc[S_BNORM2] = a[0];
@@ -266,21 +256,14 @@ __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const doubl
     }
     for (int it = 0; it < chunk && sc[S_CONV] == 0.0; ++it) {
         const double beta = sc[S_BETA], omega0 = sc[S_OMEGA];
-        FOR_ROWS if (in) {
-            if (ONE) p = __fma_rn(beta, __fma_rn(-omega0, v, p), r);
-            S.p[i] = ONE ? p : __fma_rn(beta, __fma_rn(-omega0, S.v[i], S.p[i]), S.r[i]);
-        }
+        if (in) S.p[i] = p = __fma_rn(beta, __fma_rn(-omega0, v, p), r);
         if (!grid_barrier(G)) return;
-        FOR_ROWS {   // v = A p, (rh, v) -> alpha
-            double q[2] = {0.0, 0.0};
-            if (in) {
-                const double vi = row(vb, S.p);
-                if (ONE) v = vi;
-                else S.v[i] = vi;
-                q[0] = __dmul_rn(ONE ? rh : S.rh[i], vi);
-            }
-            partial(vb, q);
+        double q[2] = {0.0, 0.0};
+        if (in) {   // v = A p, (rh, v) -> alpha
+            v = row(S.p);
+            q[0] = __dmul_rn(rh, v);
         }
+        partial(q);
         if (!total(a)) return;
         if (t == 0) {
             if (a[0] == 0.0 || !isfinite(a[0])) {
@@ -292,22 +275,15 @@ __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const doubl
         }
         __syncthreads();
         const double alpha = sc[S_ALPHA];
-        FOR_ROWS if (in) {
-            if (ONE) s = __fma_rn(-alpha, v, r);
-            S.s[i] = ONE ? s : __fma_rn(-alpha, S.v[i], S.r[i]);
-        }
+        if (in) S.s[i] = s = __fma_rn(-alpha, v, r);
         if (!grid_barrier(G)) return;
-        FOR_ROWS {   // t = A s, (t, s) and (t, t) -> omega
-            double q[2] = {0.0, 0.0};
-            if (in) {
-                const double ti = row(vb, S.s);
-                if (ONE) w = ti;
-                else S.t[i] = ti;
-                q[0] = __dmul_rn(ti, ONE ? s : S.s[i]);
-                q[1] = __dmul_rn(ti, ti);
-            }
-            partial(vb, q);
+        q[0] = q[1] = 0.0;
+        if (in) {   // t = A s, (t, s) and (t, t) -> omega
+            w = row(S.s);
+            q[0] = __dmul_rn(w, s);
+            q[1] = __dmul_rn(w, w);
         }
+        partial(q);
         if (!total(a)) return;
         if (t == 0) {
             sc[S_OMEGA] = (a[1] != 0.0) ? a[0] / a[1] : 0.0;
@@ -316,20 +292,14 @@ __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const doubl
         __syncthreads();
         const double omega = sc[S_OMEGA];
         if (t == NT - 1) ratio = alpha / omega;   // (beside the other warps; a division takes 500 cycles)
-        FOR_ROWS {   // x, r; (rh, r) and (r, r) -> beta, the stopping test
-            double q[2] = {0.0, 0.0};
-            if (in) {
-                const double si = ONE ? s : S.s[i];
-                if (ONE) xi = __fma_rn(omega, s, __fma_rn(alpha, p, xi));
-                else x[i] = __fma_rn(omega, si, __fma_rn(alpha, S.p[i], x[i]));
-                const double ri = __fma_rn(-omega, ONE ? w : S.t[i], si);
-                if (ONE) r = ri;
-                else S.r[i] = ri;
-                q[0] = __dmul_rn(ONE ? rh : S.rh[i], ri);
-                q[1] = __dmul_rn(ri, ri);
-            }
-            partial(vb, q);
+        q[0] = q[1] = 0.0;
+        if (in) {   // x, r; (rh, r) and (r, r) -> beta, the stopping test
+            xi = __fma_rn(omega, s, __fma_rn(alpha, p, xi));
+            r = __fma_rn(-omega, w, s);
+            q[0] = __dmul_rn(rh, r);
+            q[1] = __dmul_rn(r, r);
         }
+        partial(q);
         if (!total(a)) return;
         if (t == 0) {
             sc[S_BETA] = __dmul_rn(a[0] / sc[S_RHO], ratio);
@@ -342,27 +312,179 @@ __global__ void __launch_bounds__(BS_STATIC_THREADS) ks_solve(Csr A, const doubl
         }
         __syncthreads();
     }
-    if (ONE && in1) {
-        x[ir] = xi;
-        S.r[ir] = r;
-        S.v[ir] = v;
+    if (in) {
+        x[i] = xi;
+        S.r[i] = r;
+        S.v[i] = v;
     }
     if (sc[S_CONV] != 0.0) {   // the true residual
         if (!grid_barrier(G)) return;
-        FOR_ROWS {
-            double q[2] = {0.0, 0.0};
-            if (in) {
-                const double ri = b[i] - row(vb, x);
-                q[0] = __dmul_rn(ri, ri);
-            }
-            partial(vb, q);
+        double q[2] = {0.0, 0.0};
+        if (in) {
+            const double ri = b[i] - row(x);
+            q[0] = __dmul_rn(ri, ri);
         }
+        partial(q);
         if (!total(a)) return;
         if (t == 0) sc[S_RTRUE2] = a[0];
     }
-#undef FOR_ROWS
     __syncthreads();
     if (blockIdx.x == 0 && t < 16) S.sc[t] = sc[t];
+}
+
+// ---- launch per phase: where the cooperative launch is not to be had (fewer
+// resident blocks than row blocks: a partition of the device, a green context).
+// It resumes from what ks_solve leaves between its launches (r, rhat, p, v, the
+// scalars), and gives the same iterates.
+__device__ __forceinline__ double csr_row(const Csr& A, const double* __restrict__ u, int i) {
+    double acc = 0.0;
+    for (int e = A.rp[i]; e < A.rp[i + 1]; ++e) acc += A.val[e] * u[A.col[e]];
+    return acc;
+}
+
+template <int NV>
+__device__ __forceinline__ void block_partials(double (&v)[NV], double* part) {
+    __shared__ double sh[NV * 32];
+    block_sum<NV>(v, sh);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) part[blockIdx.x * BS_STATIC_NPART + q] = v[q];
+}
+
+__device__ __forceinline__ bool done(const Scr& S) { return S.sc[S_CONV] != 0.0; }
+
+__global__ void ks_init(Csr A, const double* __restrict__ b, const double* __restrict__ x, double* base) {
+    const Scr S = carve(base);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double q[2] = {0.0, 0.0};
+    if (i < A.n) {
+        const double ri = b[i] - csr_row(A, x, i);
+        S.r[i] = ri;
+        S.rh[i] = ri;
+        S.p[i] = 0.0;
+        S.v[i] = 0.0;
+        q[0] = b[i] * b[i];
+        q[1] = ri * ri;
+    }
+    block_partials<2>(q, S.part);
+}
+
+// single block: sum the partials in block order and update the scalars
+__global__ void ks_reduce(int nblk, int phase, double tol, int maxit, double* base) {
+    const Scr S = carve(base);
+    // the host launches iterations in groups: once a solve has converged the
+    // iteration phases of the rest of the group leave every scalar (and the
+    // iteration count) as they are; the flag is read by the whole block, so
+    // the early return is uniform
+    if (phase >= 1 && phase <= 3 && S.sc[S_CONV] != 0.0) return;
+    __shared__ double sh[3 * 32];
+    double a[3] = {0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x)
+        for (int q = 0; q < 3; ++q) a[q] += S.part[b * BS_STATIC_NPART + q];
+    block_sum<3>(a, sh);
+    if (threadIdx.x != 0) return;
+    double* sc = S.sc;
+    if (phase == 0) {   // init: (b,b), (r,r)
+        sc[S_BNORM2] = a[0];
+        sc[S_RNORM2] = a[1];
+        sc[S_RHO] = a[1];
+        sc[S_ALPHA] = 1.0;
+        sc[S_OMEGA] = 1.0;
+        sc[S_BETA] = 0.0;
+        sc[S_ITERS] = 0.0;
+        sc[S_BREAK] = 0.0;
+        sc[S_CONV] = (a[0] == 0.0 || a[1] <= tol * tol * a[0]) ? 1.0 : 0.0;
+    } else if (phase == 1) {   // (rhat, v) -> alpha
+        if (a[0] == 0.0 || !isfinite(a[0])) {
+            sc[S_BREAK] = 1.0;
+            sc[S_ALPHA] = 0.0;
+        } else {
+            sc[S_ALPHA] = sc[S_RHO] / a[0];
+        }
+    } else if (phase == 2) {   // (t,s), (t,t) -> omega
+        sc[S_OMEGA] = (a[1] != 0.0) ? a[0] / a[1] : 0.0;
+        if (a[1] == 0.0) sc[S_BREAK] = 1.0;
+    } else if (phase == 3) {   // (rhat, r), (r,r) -> beta, convergence
+        sc[S_BETA] = (a[0] / sc[S_RHO]) * (sc[S_ALPHA] / sc[S_OMEGA]);
+        sc[S_RHO] = a[0];
+        sc[S_RNORM2] = a[1];
+        sc[S_ITERS] += 1.0;
+        const bool conv = a[1] <= tol * tol * sc[S_BNORM2] || !isfinite(a[1]) || sc[S_BREAK] != 0.0 ||
+                          sc[S_ITERS] >= (double)maxit;
+        sc[S_CONV] = conv ? 1.0 : 0.0;
+    } else {   // true residual
+        sc[S_RTRUE2] = a[0];
+    }
+}
+
+__global__ void ks_p(Csr A, double* base) {
+    const Scr S = carve(base);
+    if (done(S)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= A.n) return;
+    S.p[i] = S.r[i] + S.sc[S_BETA] * (S.p[i] - S.sc[S_OMEGA] * S.v[i]);
+}
+
+__global__ void ks_v(Csr A, double* base) {
+    const Scr S = carve(base);
+    if (done(S)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double q[1] = {0.0};
+    if (i < A.n) {
+        const double vi = csr_row(A, S.p, i);
+        S.v[i] = vi;
+        q[0] = S.rh[i] * vi;
+    }
+    block_partials<1>(q, S.part);
+}
+
+__global__ void ks_s(Csr A, double* base) {
+    const Scr S = carve(base);
+    if (done(S)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= A.n) return;
+    S.s[i] = S.r[i] - S.sc[S_ALPHA] * S.v[i];
+}
+
+__global__ void ks_t(Csr A, double* base) {
+    const Scr S = carve(base);
+    if (done(S)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double q[2] = {0.0, 0.0};
+    if (i < A.n) {
+        const double ti = csr_row(A, S.s, i);
+        S.t[i] = ti;
+        q[0] = ti * S.s[i];
+        q[1] = ti * ti;
+    }
+    block_partials<2>(q, S.part);
+}
+
+__global__ void ks_x(Csr A, double* __restrict__ x, double* base) {
+    const Scr S = carve(base);
+    if (done(S)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double q[2] = {0.0, 0.0};
+    if (i < A.n) {
+        const double a = S.sc[S_ALPHA], w = S.sc[S_OMEGA];
+        x[i] = x[i] + a * S.p[i] + w * S.s[i];
+        const double ri = S.s[i] - w * S.t[i];
+        S.r[i] = ri;
+        q[0] = S.rh[i] * ri;
+        q[1] = ri * ri;
+    }
+    block_partials<2>(q, S.part);
+}
+
+__global__ void ks_true(Csr A, const double* __restrict__ b, const double* __restrict__ x, double* base) {
+    const Scr S = carve(base);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double q[1] = {0.0};
+    if (i < A.n) {
+        const double ri = b[i] - csr_row(A, x, i);
+        q[0] = ri * ri;
+    }
+    block_partials<1>(q, S.part);
 }
 
 // device address of the scratch array, looked up once per device
@@ -385,9 +507,10 @@ int scratch_for_current_device(double** out) {
 
 }  // namespace
 
-extern "C" int bs_bicgstab_csr_noalloc(int32_t n, const int32_t* d_row_ptr, const int32_t* d_col,
-                                       const double* d_val, const double* d_b, double* d_x, double tol,
-                                       int32_t maxit, void* stream, int32_t* iters, double* relres) {
+// form 0: one cooperative launch where it is to be had; 1: the launches per phase
+static int solve_noalloc(int32_t n, const int32_t* d_row_ptr, const int32_t* d_col, const double* d_val,
+                         const double* d_b, double* d_x, double tol, int32_t maxit, void* stream, int32_t* iters,
+                         double* relres, int form) {
     if (n <= 0 || !d_row_ptr || !d_col || !d_val || !d_b || !d_x || maxit <= 0 || !(tol >= 0.0)) return BS_E_ARG;
     if (n > BS_STATIC_MAX_ROWS) return BS_E_CAPACITY;
     double* base = nullptr;
@@ -400,37 +523,75 @@ extern "C" int bs_bicgstab_csr_noalloc(int32_t n, const int32_t* d_row_ptr, cons
     int dev = 0, sms = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return BS_E_CUDA;
-    const int cap = nb <= sms ? 17000 : 8000, smem = cap * 12;
-    auto most = [&](auto kernel) {   // resident blocks of the kernel
-        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-               cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, BS_STATIC_THREADS, smem) == cudaSuccess;
-    };
-    if (!most(ks_solve<true>)) return BS_E_CUDA;
-    const bool one = (long)per * sms >= nb;
-    if (!one && !most(ks_solve<false>)) return BS_E_CUDA;
-    int grid = (int)std::min<long>(nb, (long)per * sms);
-    if (grid < 1) return BS_E_CUDA;
+    const int most = 17000, cap = nb <= sms ? most : 8000, smem = cap * 12;
+    // (the kernel's limit is the same on every call: calls of other sizes may be running)
+    bool coop = form == 0 &&
+                cudaFuncSetAttribute(ks_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, most * 12) == cudaSuccess &&
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ks_solve, BS_STATIC_THREADS, smem) == cudaSuccess;
+    if (form == 0 && !coop) cudaGetLastError();
+    if ((long)per * sms < nb) coop = false;
     double sc[32];
     const Scr S = carve(base);
     int first = 1, chunk = BS_STATIC_CHUNK;
-    while (true) {
-        if (cudaMemsetAsync(S.sc + 24, 0, 2 * sizeof(double), st) != cudaSuccess) return BS_E_CUDA;
-        void* args[] = {(void*)&A, (void*)&d_b, (void*)&d_x, (void*)&base, (void*)&nb, (void*)&tol, (void*)&maxit,
-                        (void*)&chunk, (void*)&first, (void*)&cap};
-        if (cudaLaunchCooperativeKernel(one ? (const void*)ks_solve<true> : (const void*)ks_solve<false>, dim3(grid),
-                                        dim3(BS_STATIC_THREADS), args, smem, st) != cudaSuccess)
-            return BS_E_CUDA;
+    for (long it = 0;;) {
+        if (coop) {
+            if (cudaMemsetAsync(S.sc + 24, 0, 2 * sizeof(double), st) != cudaSuccess) return BS_E_CUDA;
+            void* args[] = {(void*)&A, (void*)&d_b, (void*)&d_x, (void*)&base, (void*)&nb, (void*)&tol, (void*)&maxit,
+                            (void*)&chunk, (void*)&first, (void*)&cap};
+            if (cudaLaunchCooperativeKernel((const void*)ks_solve, dim3(nb), dim3(BS_STATIC_THREADS), args, smem, st) !=
+                cudaSuccess) {   // (the stream's share of the device is smaller than the device)
+                cudaGetLastError();
+                coop = false;
+                continue;
+            }
+            it += chunk;
+        } else {
+            if (first) {
+                ks_init<<<nb, BS_STATIC_THREADS, 0, st>>>(A, d_b, d_x, base);
+                ks_reduce<<<1, 256, 0, st>>>(nb, 0, tol, maxit, base);
+            }
+            // check every 4 iterations; kernels of a converged solve return at once
+            for (int c = 0; c < 4; ++c, ++it) {
+                ks_p<<<nb, BS_STATIC_THREADS, 0, st>>>(A, base);
+                ks_v<<<nb, BS_STATIC_THREADS, 0, st>>>(A, base);
+                ks_reduce<<<1, 256, 0, st>>>(nb, 1, tol, maxit, base);
+                ks_s<<<nb, BS_STATIC_THREADS, 0, st>>>(A, base);
+                ks_t<<<nb, BS_STATIC_THREADS, 0, st>>>(A, base);
+                ks_reduce<<<1, 256, 0, st>>>(nb, 2, tol, maxit, base);
+                ks_x<<<nb, BS_STATIC_THREADS, 0, st>>>(A, d_x, base);
+                ks_reduce<<<1, 256, 0, st>>>(nb, 3, tol, maxit, base);
+            }
+        }
         if (cudaMemcpyAsync(sc, S.sc, sizeof(sc), cudaMemcpyDeviceToHost, st) != cudaSuccess) return BS_E_CUDA;
         if (cudaStreamSynchronize(st) != cudaSuccess) return BS_E_CUDA;
-        unsigned broken;
-        std::memcpy(&broken, sc + 25, sizeof(broken));
+        unsigned broken = 0;
+        if (coop) std::memcpy(&broken, sc + 25, sizeof(broken));
         if (broken) return BS_E_CUDA;   // a block's wait for the others ran out
-        if (sc[S_CONV] != 0.0) break;
         first = 0;
+        if (sc[S_CONV] != 0.0 || it >= maxit) break;
+    }
+    if (!coop) {
+        ks_true<<<nb, BS_STATIC_THREADS, 0, st>>>(A, d_b, d_x, base);
+        ks_reduce<<<1, 256, 0, st>>>(nb, 4, tol, maxit, base);
+        if (cudaMemcpyAsync(sc, S.sc, sizeof(sc), cudaMemcpyDeviceToHost, st) != cudaSuccess) return BS_E_CUDA;
+        if (cudaStreamSynchronize(st) != cudaSuccess) return BS_E_CUDA;
     }
     if (cudaGetLastError() != cudaSuccess) return BS_E_CUDA;
     if (iters) *iters = (int32_t)sc[S_ITERS];
     if (relres) *relres = sc[S_BNORM2] > 0.0 ? std::sqrt(sc[S_RTRUE2] / sc[S_BNORM2]) : std::sqrt(sc[S_RTRUE2]);
     const bool ok = sc[S_BNORM2] == 0.0 || sc[S_RNORM2] <= tol * tol * sc[S_BNORM2];
     return ok ? BS_OK : BS_E_NOTCONV;
+}
+
+extern "C" int bs_bicgstab_csr_noalloc(int32_t n, const int32_t* d_row_ptr, const int32_t* d_col,
+                                       const double* d_val, const double* d_b, double* d_x, double tol,
+                                       int32_t maxit, void* stream, int32_t* iters, double* relres) {
+    return solve_noalloc(n, d_row_ptr, d_col, d_val, d_b, d_x, tol, maxit, stream, iters, relres, 0);
+}
+
+// the launches per phase on any device (not in the public header: their tests)
+extern "C" int bs_bicgstab_csr_noalloc_phases(int32_t n, const int32_t* d_row_ptr, const int32_t* d_col,
+                                              const double* d_val, const double* d_b, double* d_x, double tol,
+                                              int32_t maxit, void* stream, int32_t* iters, double* relres) {
+    return solve_noalloc(n, d_row_ptr, d_col, d_val, d_b, d_x, tol, maxit, stream, iters, relres, 1);
 }

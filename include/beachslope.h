@@ -451,6 +451,10 @@ int bs_fgmres_csr(int32_t n, const int32_t* row_ptr, const int32_t* col, const d
  * residual ||b - A x|| / ||b|| after the last iteration; the convergence flag
  * is read back every 256 iterations (the call waits for `stream` there), so
  * the call must not be made on a stream that is being captured into a graph.
+ * The iterations run in one cooperative launch of n / 256 blocks (up to 204 KB
+ * of shared memory each): beside other streams' kernels it starts when theirs
+ * leave room for all of its blocks.  Where the device refuses that launch (a
+ * partition or green context with too few SMs) each phase is its own launch.
  * `stream` is a cudaStream_t (NULL: the default stream). */
 int bs_bicgstab_csr_noalloc(int32_t n, const int32_t* d_row_ptr, const int32_t* d_col, const double* d_val,
                             const double* d_b, double* d_x, double tol, int32_t maxit, void* stream,
