@@ -87,8 +87,10 @@ struct bs_ctx {
     // mixed form's cycle; the Krylov solve and its stopping test stay FP64)
     int mg_fp32 = 0;
     // threads per block of the neighbour sweeps and of the particle-level
-    // multigrid kernels (options "sweep_tpb", "mg0_tpb"; the autotuner picks them)
+    // multigrid kernels (options "sweep_tpb", "mg0_tpb"; the autotuner picks them);
+    // sweep_set: the size was asked for, and runs as asked
     int sweep_tpb = BS_THREADS, mg0_tpb = BS_THREADS;
+    bool sweep_set = false;
     // exact coarse solve (option "mg_exact"): the scenes' exactly solved levels
     MgExact mgexact{};
     // captured production steps (one CUDA graph per step, loops on the device):
@@ -199,6 +201,19 @@ int fg_ensure(bs_ctx* ctx) {
 // precision of the multigrid preconditioner's cycle (its setup, matrix copy and level arrays)
 int mg_prec_of(const bs_ctx* c) { return (c->precision == BS_PREC_MIXED || c->mg_fp32) ? BS_PREC_MIXED : BS_PREC_FP64; }
 
+// Threads per block of the neighbour sweeps: the size asked for (option
+// "sweep_tpb"); else 256, and for a small scene blocks small enough for two on
+// each SM: its FP64 pair arithmetic is bound by each SM's pipe (13,681 rows of 30
+// neighbours on 54 SMs in blocks of 256, on all in blocks of 32: search 477 and
+// 333 us, int_vel 228 and 171; 15 k rows in mixed precision take the same either
+// way).
+int sweep_threads(const bs_ctx* c) {
+    int t = c->sweep_tpb;
+    if (!c->sweep_set)
+        while (t > 32 && (long)c->nblk_total * (BS_THREADS / t) < 2L * c->sm_count) t /= 2;
+    return t;
+}
+
 bs::Launch launch_of(bs_ctx* c) {
     bs::Launch L;
     L.stream = c->stream;
@@ -214,12 +229,7 @@ bs::Launch launch_of(bs_ctx* c) {
     L.mgchip_cs = c->mgchip_cs;
     L.mgchip_smem = c->mgchip_smem;
     L.mgsub_cs = c->mgsub_cs;
-    L.sweep_tpb = c->sweep_tpb;
-    // A small scene's sweeps in blocks small enough for two on each SM: its FP64
-    // pair arithmetic is bound by each SM's pipe (13,681 rows of 30 neighbours on
-    // 54 SMs in blocks of 256, on all in blocks of 32: search 477 and 333 us, int_vel
-    // 228 and 171; 15 k rows in mixed precision take the same either way).
-    while (L.sweep_tpb > 32 && (long)c->nblk_total * (BS_THREADS / L.sweep_tpb) < 2L * c->sm_count) L.sweep_tpb /= 2;
+    L.sweep_tpb = sweep_threads(c);
     L.mg0_tpb = c->mg0_tpb;
     L.exact = &c->mgexact;
     return L;
@@ -1369,8 +1379,10 @@ int bs_set_option(bs_ctx* ctx, const char* name, double value) {
         M.exact = (int)value;
         if (!ctx->mglev.empty()) mg_tables(ctx);
     }
-    else if ((k == "sweep_tpb" || k == "mg0_tpb") && (value == 64 || value == 128 || value == 256))
+    else if ((k == "sweep_tpb" || k == "mg0_tpb") && (value == 64 || value == 128 || value == 256)) {
         (k == "sweep_tpb" ? ctx->sweep_tpb : ctx->mg0_tpb) = (int)value;
+        if (k == "sweep_tpb") ctx->sweep_set = true;
+    }
     else if (k == "step_graph" && (value == 0 || value == 1)) {
         ctx->step_graph_on = (int)value;
         ctx->step_graph_broken = false;
@@ -1407,6 +1419,7 @@ int bs_get_option(bs_ctx* ctx, const char* name, double* value) {
     else if (k == "ppe_restart") *value = ctx->prm[0].ppe_restart;
     else if (k == "mg_exact") *value = M.exact;
     else if (k == "sweep_tpb") *value = ctx->sweep_tpb;
+    else if (k == "sweep_tpb_used") *value = sweep_threads(ctx);
     else if (k == "mg0_tpb") *value = ctx->mg0_tpb;
     else if (k == "step_graph") *value = ctx->step_graph_on && !ctx->step_graph_broken;
     else if (k == "step_graph_steps") *value = (double)ctx->graph_steps;
@@ -1884,7 +1897,7 @@ std::vector<unsigned char> step_key(const bs_ctx* c, int flags) {
     const int v[] = {flags, c->precision, c->prm[0].ppe_solver, c->prm[0].ppe_restart, c->prm[0].ppe_precond,
                      c->prm[0].mixed_max_outer, max_ppe_maxit(c), c->mgsub_on, c->mgsub_level, c->mgsub_cs,
                      c->fg_df_on, c->disp_ready ? 1 : 0, any_scalar_on(c) ? 1 : 0, c->nblk_total,
-                     c->sweep_tpb, c->mg0_tpb, c->mg_fp32, c->mgtail_level, c->mgchip_cs, c->mgchip_smem};
+                     sweep_threads(c), c->mg0_tpb, c->mg_fp32, c->mgtail_level, c->mgchip_cs, c->mgchip_smem};
     key_put(k, v);
     for (const auto& m : c->mglev) key_put(k, m);
     k.insert(k.end(), c->mgneed.begin(), c->mgneed.end());

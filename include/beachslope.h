@@ -348,10 +348,12 @@ int bs_write_combined(struct bs_ctx* ctx, int32_t scene, const char* fluid_path,
  * bit-identical to the separate launches), "sweep_tpb" /
  * "mg0_tpb" (64, 128 or 256 threads per block of the neighbour sweeps / of
  * the particle-level multigrid kernels; every row is computed the same way
- * whatever the block size), "step_graph" (0/1, default 1: each bs_step is
+ * whatever the block size; until "sweep_tpb" is set, scenes too small for two
+ * blocks of 256 on each SM take smaller ones, down to 32: "sweep_tpb_used" reads
+ * the size in use), "step_graph" (0/1, default 1: each bs_step is
  * one captured CUDA graph with the loops on the device);
- * bs_get_option also reads "mg_levels", "mg_sub_level", "mg_tail_level", "step_graph_steps"
- * and "step_graph_cached". */
+ * bs_get_option also reads "mg_levels", "mg_sub_level", "mg_tail_level",
+ * "sweep_tpb_used", "step_graph_steps" and "step_graph_cached". */
 int bs_set_option(struct bs_ctx* ctx, const char* name, double value);
 int bs_get_option(struct bs_ctx* ctx, const char* name, double* value);
 
