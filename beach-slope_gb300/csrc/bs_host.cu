@@ -2185,12 +2185,15 @@ static int krylov_csr(int solver, int32_t n, const int32_t* row_ptr, const int32
     CK(cudaMemcpy(D.aval, aval.data(), sizeof(double) * E, cudaMemcpyHostToDevice));
     ctx->assembled = true;
     D.fg_df = 0;
-    // Columns and iterations per graph launch and read of the converged count (4 us of
-    // a column's or an iteration's time): FGMRES 10.2 -> 7.8 ms at 60,025 rows,
-    // BiCGStab 4.43 -> 4.13 at 2,500; what a chunk runs past the end are empty
-    // launches, five per iteration of BiCGStab: 100 us, more than the few iterations
-    // of a system below 1,024 rows gain.
-    const int chunk = solver == BS_SOLVER_FGMRES || n >= 1024 ? 8 : 1;
+    // Columns or iterations per graph launch and read of the converged count.  One
+    // by one the read costs 4 us of each; what a chunk runs past the end of a cycle
+    // or solve are empty launches (3 a column, 5 an iteration of BiCGStab, 2 us
+    // each).  Whole calls at chunks of 1, 4 and 8, ms: FGMRES, 9,801 rows, restart
+    // 150: 8.51 7.79 7.79; restart 4: 14.96 12.74 13.72; restart 1: 3.90 4.19 4.57;
+    // 60 rows, 5 columns: 1.44 1.47 1.52, 9: 1.58 1.58 1.63, 41: 2.79 2.56 2.59.
+    // BiCGStab, 9,801 rows, 5 iterations: 2.55 2.60 2.65, 41: 3.86 3.74 3.79; 60
+    // rows, 9 iterations: 1.51 1.54 1.61.
+    const int chunk = solver == BS_SOLVER_FGMRES ? std::min(restart, 4) : n >= 1024 ? 4 : 1;
     if (solver == BS_SOLVER_FGMRES)
         bs::solve_fgmres(D, launch_of(ctx), maxit, chunk, 0, BS_PREC_FP64, ctx->d_nconv, ctx->h_pinned, ctx->evsync);
     else

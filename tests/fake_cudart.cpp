@@ -168,7 +168,7 @@ cudaError_t cudaMemset(void* d, int v, size_t n) { return std::memset(d, v, n), 
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return std::memset(d, v, n), cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { return *f = room - used, *t = room, cudaSuccess; }
 
-// ---- streams, events, graphs (captures are refused: the library then launches kernel by kernel)
+// ---- streams, events, graphs (what is captured is recorded once, at the capture; no conditional nodes)
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return *s = (cudaStream_t)&token, cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
@@ -180,17 +180,19 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.0f, cudaSuccess; }
-cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return ret(cudaErrorNotSupported); }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) { return *g = (cudaGraph_t)&token, cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+    return *e = (cudaGraphExec_t)&token, cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t fake_unsupported() { return ret(cudaErrorNotSupported); }
 }
 #define UNSUPPORTED(name) asm(".globl " #name "\n.set " #name ", fake_unsupported")
 UNSUPPORTED(cudaGraphAddNode);
 UNSUPPORTED(cudaGraphConditionalHandleCreate);
-UNSUPPORTED(cudaGraphDestroy);
-UNSUPPORTED(cudaGraphExecDestroy);
-UNSUPPORTED(cudaGraphInstantiate);
-UNSUPPORTED(cudaGraphLaunch);
 UNSUPPORTED(cudaStreamBeginCaptureToGraph);
-UNSUPPORTED(cudaStreamEndCapture);
 UNSUPPORTED(cudaStreamGetCaptureInfo);
 UNSUPPORTED(cudaStreamUpdateCaptureDependencies);
