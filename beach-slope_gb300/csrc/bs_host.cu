@@ -80,6 +80,7 @@ struct bs_ctx {
     // launches): the level it starts at (0: off or no level qualifies), the
     // blocks per cluster and the shared memory of a block
     int mgtail_on = 1, mgtail_level = 0, mgchip_cs = 1, mgchip_smem = 0;
+    int mgchip_lose = -1;        // (tests) the block of each cluster that gives up its wait
     size_t chip_img_bytes = 0;   // size of D.mg.chip_img
     // FGMRES basis as double-float (hi, lo) FP32 pairs in the preconditioned mixed solve
     int fg_df_on = 1;
@@ -228,6 +229,7 @@ bs::Launch launch_of(bs_ctx* c) {
     L.mgtail = c->mgtail_level;
     L.mgchip_cs = c->mgchip_cs;
     L.mgchip_smem = c->mgchip_smem;
+    L.mgchip_lose = c->mgchip_lose;
     L.mgsub_cs = c->mgsub_cs;
     L.sweep_tpb = sweep_threads(c);
     L.mg0_tpb = c->mg0_tpb;
@@ -1396,6 +1398,16 @@ int bs_set_option(bs_ctx* ctx, const char* name, double value) {
     return 0;
 }
 
+// (not in the public header: tests of the on-chip levels' give-up path)  Block
+// `rank` of each cluster gives up its wait for its constants at once; -1: none.
+int bs_mg_chip_lose(bs_ctx* ctx, int32_t rank) {
+    if (!ctx) return BS_E_ARG;
+    ctx->mgchip_lose = rank;
+    sg_clear(ctx);
+    ctx->graph.valid = false;
+    return 0;
+}
+
 int bs_get_option(bs_ctx* ctx, const char* name, double* value) {
     if (!ctx || !name || !value) return BS_E_ARG;
     const MgDev& M = ctx->D.mg;
@@ -1414,6 +1426,7 @@ int bs_get_option(bs_ctx* ctx, const char* name, double* value) {
     else if (k == "fg_df") *value = ctx->fg_df_on;
     else if (k == "mg_tail") *value = ctx->mgtail_on;
     else if (k == "mg_tail_level") *value = ctx->mgtail_level;
+    else if (k == "mg_tail_blocks") *value = ctx->mgtail_level ? ctx->mgchip_cs : 0;
     else if (k == "mg_fp32") *value = ctx->mg_fp32;
     else if (k == "mg_sub_level") *value = ctx->mgsub_level;
     else if (k == "ppe_restart") *value = ctx->prm[0].ppe_restart;
@@ -1897,7 +1910,8 @@ std::vector<unsigned char> step_key(const bs_ctx* c, int flags) {
     const int v[] = {flags, c->precision, c->prm[0].ppe_solver, c->prm[0].ppe_restart, c->prm[0].ppe_precond,
                      c->prm[0].mixed_max_outer, max_ppe_maxit(c), c->mgsub_on, c->mgsub_level, c->mgsub_cs,
                      c->fg_df_on, c->disp_ready ? 1 : 0, any_scalar_on(c) ? 1 : 0, c->nblk_total,
-                     sweep_threads(c), c->mg0_tpb, c->mg_fp32, c->mgtail_level, c->mgchip_cs, c->mgchip_smem};
+                     sweep_threads(c), c->mg0_tpb, c->mg_fp32, c->mgtail_level, c->mgchip_cs, c->mgchip_smem,
+                     c->mgchip_lose};
     key_put(k, v);
     for (const auto& m : c->mglev) key_put(k, m);
     k.insert(k.end(), c->mgneed.begin(), c->mgneed.end());

@@ -494,6 +494,11 @@ __device__ __forceinline__ void st_rank(unsigned p, int rank, float v) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(p), "r"(rank));
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
+__device__ __forceinline__ void st_rank(unsigned p, int rank, unsigned v) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(p), "r"(rank));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
 __device__ __forceinline__ void st_rank(unsigned p, int rank, double v) {
     unsigned a;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(p), "r"(rank));
@@ -591,6 +596,7 @@ struct MgSub {
 // and the first cell on each level.
 #define BS_CHIP_SMEM (200 * 1024)    // most shared memory a block of it takes
 struct MgChip {
+    int lose;                         // the rank whose wait for its constants gives up at once (-1: none; tests)
     int l0, nops, cs, stride;         // stride: bytes of a block's constants in MgDev::chip_img (its shared memory)
     unsigned char op[BS_MG_MAXOPS], lv[BS_MG_MAXOPS], acc[BS_MG_MAXOPS];
     int nx[BS_MG_MAXS], ny[BS_MG_MAXS], lev[BS_MG_MAXS], off[BS_MG_SUBL][BS_MG_MAXS];
@@ -609,6 +615,7 @@ struct Launch {
     int mgsub_level, mgsub_cs;     // first level of the clustered subtree (0: per-level launches), CTAs per cluster
     int mgtail;                    // level whose visits run on chip, everything below included (0: none)
     int mgchip_cs, mgchip_smem;    // ... blocks per cluster and bytes of shared memory per block
+    int mgchip_lose;               // MgChip::lose
     int sweep_tpb;                 // threads per block of the neighbour sweeps (32, 64, 128 or 256)
     int mg0_tpb;                   // threads per block of the particle-level multigrid kernels
     const MgExact* exact;          // the scenes' exactly solved levels (when D.mg.exact)

@@ -769,6 +769,19 @@ __device__ __forceinline__ void chip_dots(const T (&a)[9][4], const T (&W)[4][4]
         for (int ch = 0; ch < 4; ++ch) ax[ch] += a[s][ch] * W[(ch >> 1) + s / 3][(ch & 1) + s % 3];
 }
 
+// Has the block's constants' copy landed?  (bounded: a copy that never ended
+// would hang the GPU)
+__device__ __forceinline__ bool chip_landed(unsigned bar, int tries) {
+    unsigned ok = 0;
+    for (int it = 0; it < tries && !ok; ++it)
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared.b64 p, [%1], 0; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(ok)
+                     : "r"(bar)
+                     : "memory");
+    return ok != 0;
+}
+constexpr int CHIP_TRIES = 1 << 20;
+
 template <int N>
 struct ChipInt {
     static constexpr int value = N;
@@ -781,6 +794,7 @@ __global__ void __launch_bounds__(BS_CHIP_THREADS) k_mg_chip(Dev D, __grid_const
     extern __shared__ __align__(16) unsigned char chip_smem[];
     __shared__ unsigned ops[BS_MG_MAXOPS + 1];
     __shared__ int nlist;
+    __shared__ unsigned lost;                      // a block of the cluster gave up
     __shared__ __align__(8) unsigned long long bar;
     const MgDev& M = D.mg;
     const int cs = S.cs, lg = 31 - __clz(cs);
@@ -794,7 +808,7 @@ __global__ void __launch_bounds__(BS_CHIP_THREADS) k_mg_chip(Dev D, __grid_const
     }
     // constants of the solve
     const unsigned sbar = (unsigned)__cvta_generic_to_shared(&bar), sb = (unsigned)__cvta_generic_to_shared(chip_smem);
-    const unsigned sops = (unsigned)__cvta_generic_to_shared(ops);
+    const unsigned sops = (unsigned)__cvta_generic_to_shared(ops), slost = (unsigned)__cvta_generic_to_shared(&lost);
     if (t == 0) {
         const unsigned char* img = (const unsigned char*)M.chip_img + (long)blockIdx.x * S.stride;
         const unsigned bytes = (unsigned)((rank == 0 ? S.img[k] : S.img0[k]) - S.zero[k]);
@@ -832,24 +846,24 @@ __global__ void __launch_bounds__(BS_CHIP_THREADS) k_mg_chip(Dev D, __grid_const
         for (int e = BS_CHIP_HDR / 16 + t; e < e1; e += NT)
             reinterpret_cast<float4*>(chip_smem)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    if (t == 0) lost = 0;
     if (d > 0) cluster_arrive();                   // every block of the cluster runs before remote stores
     __syncthreads();
-    {
-        bool here = false;                         // (bounded: a copy that never ended would hang the GPU)
-        for (int it = 0; it < (1 << 20) && !here; ++it) {
-            unsigned ok;
-            asm volatile(
-                "{ .reg .pred p; mbarrier.try_wait.parity.shared.b64 p, [%1], 0; selp.u32 %0, 1, 0, p; }"
-                : "=r"(ok)
-                : "r"(sbar)
-                : "memory");
-            here = ok != 0;
+    if (__syncthreads_or(!chip_landed(sbar, rank == S.lose ? 0 : CHIP_TRIES))) {
+        // Gives up, together with its cluster: the others store into this block's
+        // shared memory until the barrier behind their first operation, and leave
+        // there when they find `lost`.  Its own copy ends first.
+        chip_landed(sbar, CHIP_TRIES);
+        BS_PDL_ENTRY();
+        const bool live = !mg_skip(D, k, fg);      // (else the others leave without an operation)
+        if (d > 0) cluster_wait();
+        if (live && d > 0) {
+            if (t < cs) st_rank(slost, t, 1u);
+            cluster_arrive();
+            cluster_wait();
         }
-        if (__syncthreads_or(!here)) {
-            BS_PDL_ENTRY();
-            if (t == 0) set_err(D, k, BS_ERR_SOLVER_BREAK);
-            return;
-        }
+        if (live && t == 0) set_err(D, k, BS_ERR_SOLVER_BREAK);
+        return;
     }
     // level tables: x y z w = (R, area, sy, DV), (A, tab, Q, ny), (ncsy, left, nx, nc), (j0, esh, cols, -)
     auto lev = [&](int u, int part) { return sld_i4(sb + u * (int)sizeof(ChipLev) + part * 16); };
@@ -919,7 +933,7 @@ __global__ void __launch_bounds__(BS_CHIP_THREADS) k_mg_chip(Dev D, __grid_const
         const int ac = at + sy + SZ;                                    // the first child
         const unsigned flags = qd.y;
         const bool lpush = !solo && (flags & 16) && rank > 0, rpush = !solo && (flags & 32) && rank < cs - 1;
-        const int Q = L1.z, ny = L1.w;
+        const int ny = L1.w;
         const int4 N0 = lev(u + 1 < nl ? u + 1 : u, 0);
         auto dots = [&](const T(&W)[4][4], T(&ax)[4]) {
             if (KEEP && u == 0) {
@@ -1115,6 +1129,7 @@ __global__ void __launch_bounds__(BS_CHIP_THREADS) k_mg_chip(Dev D, __grid_const
         L1 = lev((word >> 8) & 255, 1);
         qd = t < L1.z ? sld_u2(sb + L1.y + 8 * t) : make_uint2(0, 0);
         barrier();
+        if (o == 0 && d > 0 && sld_u(slost)) return;   // (the first operation of a split visit is one of a split level)
         if (op == 0 && !solo && u + 1 >= d && rank == 0) {   // the pre-sweep of the level the others restricted to
             const int4 N3 = lev(u + 1, 2);
             for (int e = t * SZ; e < N3.x + 2 * N0.z; e += NT * SZ) {
@@ -1434,6 +1449,7 @@ void chip_args(const Dev& D, const Launch& L, int visits, MgChip& S) {
     S.l0 = L.mgtail;
     S.cs = L.mgchip_cs;
     S.stride = L.mgchip_smem;
+    S.lose = L.mgchip_lose;
     chip_ops(D, L, S.l0, visits, S);
     for (int k = 0; k < D.nscene; ++k) {
         const MgLevel& G = L.mglev[S.l0];

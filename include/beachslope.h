@@ -353,7 +353,7 @@ int bs_write_combined(struct bs_ctx* ctx, int32_t scene, const char* fluid_path,
  * the size in use), "step_graph" (0/1, default 1: each bs_step is
  * one captured CUDA graph with the loops on the device);
  * bs_get_option also reads "mg_levels", "mg_sub_level", "mg_tail_level",
- * "sweep_tpb_used", "step_graph_steps" and "step_graph_cached". */
+ * "mg_tail_blocks" (thread blocks of each of its clusters), "sweep_tpb_used", "step_graph_steps" and "step_graph_cached". */
 int bs_set_option(struct bs_ctx* ctx, const char* name, double value);
 int bs_get_option(struct bs_ctx* ctx, const char* name, double* value);
 
