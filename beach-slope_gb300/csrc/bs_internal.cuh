@@ -481,7 +481,12 @@ __device__ __forceinline__ CorrF corr_f(const Dev& D, int r) {
 }
 
 // ---- thread-block clusters
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+// (the warp's lanes arrive together, whatever branches lie before the call: every
+// lane of the warp must reach it)
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;

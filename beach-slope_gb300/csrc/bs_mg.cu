@@ -1323,6 +1323,7 @@ __global__ void k_mg_exact_apply(Dev D, __grid_constant__ const MgLevel F, int a
 // solve runs in the cluster's first block.  Every thread reaches every
 // barrier (no early exit).
 __device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();   // (the aligned form needs the warp converged)
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ unsigned cluster_size() {
