@@ -139,7 +139,10 @@ int dalloc(bs_ctx* ctx, T** p, size_t n) {
     void* q = nullptr;
     if (n == 0) n = 1;
     cudaError_t e = cudaMalloc(&q, n * sizeof(T));
-    if (e != cudaSuccess) return fail(ctx, BS_E_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // reported here, not by a later call that has nothing to do with it
+        return fail(ctx, BS_E_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     cudaMemset(q, 0, n * sizeof(T));
     ctx->allocs.push_back(q);
     ctx->alloc_bytes.push_back(n * sizeof(T));

@@ -1,0 +1,26 @@
+"""No device memory left for the on-chip multigrid levels' constants: the
+context is made all the same and takes the separate launches, and no CUDA error
+is left behind for the next call to report (host logic, no GPU)."""
+import ctypes as C
+
+from _fake_gpu import FakeGpu
+
+
+def test_no_room_for_the_chip_image(monkeypatch, tmp_path):
+    from beachslope_gb300 import scene
+    gpu = FakeGpu(monkeypatch, tmp_path)
+    p, st, gr = scene.beach_scene(dx=0.0133)
+    c = gpu.api.Context([p], [st], [gr])
+    assert c.get_option("mg_tail_level") == 1
+    total = C.c_size_t()
+    assert gpu.lib.bs_context_bytes(c.h, C.byref(total)) == 0
+    c.close()
+    gpu.lib.fake_room(total.value * 59 // 60)   # all but a part of the constants
+    c = gpu.api.Context([p], [st], [gr])
+    assert c.get_option("mg_tail_level") == 0
+    assert gpu.lib.fake_pending_error() == 0
+    c.search()   # (its launch check would report one)
+    gpu.lib.fake_room(1 << 30)
+    c.set_option("mg_tail", 1)   # room again
+    assert c.get_option("mg_tail_level") == 1
+    c.close()
