@@ -41,6 +41,7 @@ struct bs_ctx {
     int* d_nconv = nullptr;
     std::vector<void*> allocs;
     std::vector<size_t> alloc_bytes;   // size of each entry of allocs
+    bool made = false;   // bs_create has ended
     bool assembled = false;
     bool disp_ready = false;
     int max_solsteps = 1;
@@ -144,6 +145,8 @@ int dalloc(bs_ctx* ctx, T** p, size_t n) {
         return fail(ctx, BS_E_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
     cudaMemset(q, 0, n * sizeof(T));
+    // the context's streams do not wait for the null stream (bs_create waits once, at its end)
+    if (ctx->made) cudaStreamSynchronize(nullptr);
     ctx->allocs.push_back(q);
     ctx->alloc_bytes.push_back(n * sizeof(T));
     *p = (T*)q;
@@ -855,6 +858,8 @@ int bs_create(int32_t nscenes, const bs_params* params, const int32_t* capacity,
             return r2;
         }
     }
+    cudaStreamSynchronize(nullptr);   // the arrays' clearing
+    ctx->made = true;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         bs_destroy(ctx);

@@ -26,6 +26,8 @@ std::map<void*, size_t> device;          // device allocations
 size_t used = 0, room = (size_t)1 << 40;  // bytes of device memory
 cudaError_t last = cudaSuccess, refuse_coop = cudaSuccess;
 int sms = 152;
+bool clearing = false;   // a memset on the null stream that nothing has waited for
+int early = 0;           // launches while it may still run
 std::vector<cudaLaunchConfig_t> configs;
 
 cudaError_t ret(cudaError_t e) {
@@ -34,6 +36,7 @@ cudaError_t ret(cudaError_t e) {
 }
 cudaError_t record(const void* f, dim3 g, dim3 b) {
     auto it = names().find(f);
+    early += clearing;
     recs.push_back({it == names().end() ? "?" : it->second, g.x * g.y * g.z, b.x * b.y * b.z});
     return cudaSuccess;
 }
@@ -54,6 +57,7 @@ void fake_unpin(void* p) { pinned.erase((char*)p); }
 void fake_room(size_t bytes) { room = used + bytes; }
 void fake_refuse_cooperative(int e) { refuse_coop = (cudaError_t)e; }
 int fake_pending_error() { return (int)last; }
+int fake_early_launches() { return early; }
 
 // ---- module registration and launches
 void** __cudaRegisterFatBinary(void*) { return (void**)&token; }
@@ -155,7 +159,10 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
         }
     return cudaSuccess;
 }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { return std::memcpy(d, s, n), cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    clearing = false;
+    return std::memcpy(d, s, n), cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
     return std::memcpy(d, s, n), cudaSuccess;
 }
@@ -164,14 +171,20 @@ cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size
     for (size_t r = 0; r < h; ++r) std::memcpy((char*)d + r * dp, (const char*)s + r * sp, w);
     return cudaSuccess;
 }
-cudaError_t cudaMemset(void* d, int v, size_t n) { return std::memset(d, v, n), cudaSuccess; }
+cudaError_t cudaMemset(void* d, int v, size_t n) {
+    clearing = true;
+    return std::memset(d, v, n), cudaSuccess;
+}
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return std::memset(d, v, n), cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { return *f = room - used, *t = room, cudaSuccess; }
 
 // ---- streams, events, graphs (what is captured is recorded once, at the capture; no conditional nodes)
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return *s = (cudaStream_t)&token, cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    if (!s) clearing = false;   // (the library's own streams do not wait for the null stream)
+    return cudaSuccess;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return *e = (cudaEvent_t)&token, cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
