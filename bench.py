@@ -162,11 +162,11 @@ TIMED_KERNELS = ("search_effpor", "bicg_it1_spmv", "bicg_it2_spmv", "mg_l0_down"
 # DRAM bytes per launch measured by ncu over the algorithmic bytes of the same
 # launch (ncu dram__bytes_read.sum + dram__bytes_write.sum on the 0.18 M-particle beach, mixed);
 # the traffic grows with the nonzeros and rows, so the ratio scales it to the
-# bench's workload.  k_it2_64 has k_it1_64's access pattern.  fg_arnoldi_spmv:
-# every launch of seven solves of the double-float form (k_fg_arn1_df) the
-# mixed bench times.
-TRAFFIC_RATIO = {"search_effpor": 0.46, "bicg_it1_spmv": 0.99, "bicg_it2_spmv": 0.99,
-                 "mg_l0_down": 0.99, "mg_l0_up": 0.93, "fg_arnoldi_spmv": 0.90, "fg_project": 0.97}
+# bench's workload.  k_it2_64 has k_it1_64's access pattern.  fg_arnoldi_spmv and
+# fg_project: every launch of seven solves of the double-float form
+# (k_fg_arn1_df with k_fg_fin, k_fg_arn2_df) the mixed bench times.
+TRAFFIC_RATIO = {"search_effpor": 0.56, "bicg_it1_spmv": 0.99, "bicg_it2_spmv": 0.99,
+                 "mg_l0_down": 0.95, "mg_l0_up": 0.89, "fg_arnoldi_spmv": 0.96, "fg_project": 0.98}
 
 
 def fg_columns(iters, restart):
@@ -180,12 +180,13 @@ def fg_columns(iters, restart):
     return tot
 
 
-def algorithmic_bytes(ctx, kernel, precision, basis_reads=None):
+def algorithmic_bytes(ctx, kernel, precision, basis_reads=None, df=False):
     """Compulsory HBM bytes of one launch over all scenes (neighbour-vector
     gathers counted as on-chip hits; every other operand read or written once).
     w = width of the per-pair and matrix values (8 FP64, 4 mixed).  For the
     FGMRES column kernels, basis_reads = the mean number of basis vectors a
-    launch reads (j+1 at column j)."""
+    launch reads (j+1 at column j), df = the double-float form, which reads the
+    preconditioned vector in FP32."""
     w = 4 if precision == "mixed" else 8
     tot = 0.0
     for s in range(ctx.nscenes):
@@ -193,7 +194,7 @@ def algorithmic_bytes(ctx, kernel, precision, basis_reads=None):
         nnz, n = float(c.sum()), float(len(c))
         if kernel == "fg_arnoldi_spmv":
             # SpMV (FP64 values + index; diag, count, input, output) + v_j + Z_j write + basis reads
-            tot += nnz * (8 + 4) + n * (8 + 4 + 8 + 8) + n * (8 + 8) + basis_reads * n * 8
+            tot += nnz * (8 + 4) + n * (8 + 4 + (4 if df else 8) + 8) + n * (8 + 8) + basis_reads * n * 8
         elif kernel == "fg_project":
             tot += n * (8 + 8) + basis_reads * n * 8
         elif kernel in ("bicg_it1_spmv", "bicg_it2_spmv"):
@@ -291,7 +292,9 @@ def run_ours(args, D):
     cands = [(k, v[0], v[1]) for k, v in kt.items() if k in TIMED_KERNELS and v[0]]
     if cands:
         name, cnt, tms = max(cands, key=lambda t: t[2])
-        alg = algorithmic_bytes(ctx, name, args.precision, basis_reads=fg_reads / max(fg_launches, 1))
+        df = (args.precision == "mixed" and int(ctx.get_option("ppe_solver")) == abi.SOLVER_FGMRES
+              and int(ctx.get_option("fg_df")) == 1 and P[0].ppe_precond == 1)
+        alg = algorithmic_bytes(ctx, name, args.precision, basis_reads=fg_reads / max(fg_launches, 1), df=df)
         avg_s = tms / cnt / 1e3
         pk, src = peaks()
         achieved = alg / avg_s / 1e9
@@ -306,8 +309,6 @@ def run_ours(args, D):
                            "share_of_step": round(tms / ms_timed, 3),
                            "note": "durations from a second pass of the same steps with per-launch events",
                            "timed_kernels": {k: {"launches": v[0], "ms": round(v[1], 3)} for k, v in kt.items()}}
-        df = (args.precision == "mixed" and int(ctx.get_option("ppe_solver")) == abi.SOLVER_FGMRES
-              and int(ctx.get_option("fg_df")) == 1 and P[0].ppe_precond == 1)
         fl = fp64_flops(ctx, name, fg_reads / max(fg_launches, 1), df)
         if fl:
             f64pk = fp64_peak()
@@ -318,7 +319,7 @@ def run_ours(args, D):
             if df:
                 out["roofline"]["fp64"]["note"] = ("basis dots, projection and off-diagonal SpMV in "
                                                    "double-float on the FP32 pipe")
-        out["step_roofline"] = step_roofline(ctx, kt, fg_reads, fg_launches, args, ms_timed, pk, src)
+        out["step_roofline"] = step_roofline(ctx, kt, fg_reads, fg_launches, args, ms_timed, pk, src, df)
     state = ctx.download(0)
     ctx.close()
     if not args.no_e2e:
@@ -351,7 +352,7 @@ def sweep_bytes_per_particle(K, precision):
     return SWEEP_POS_WORDS * 8 + SWEEP_W_WORDS * w + 16 + SWEEP_LIST_READS * 4 * K + K + (K + 1) * 12
 
 
-def step_roofline(ctx, kt, fg_reads, fg_launches, args, ms_timed, pk, src):
+def step_roofline(ctx, kt, fg_reads, fg_launches, args, ms_timed, pk, src, df=False):
     """Whole-step roofline: the algorithmic bytes of one step (the sweeps per
     particle from sweep_bytes_per_particle, plus the solver kernels' launches
     in the event-timed pass at their per-launch algorithmic bytes) over the
@@ -364,7 +365,7 @@ def step_roofline(ctx, kt, fg_reads, fg_launches, args, ms_timed, pk, src):
         cnt = kt.get(name, (0, 0.0))[0]
         if cnt:
             solver += cnt * algorithmic_bytes(ctx, name, args.precision,
-                                              basis_reads=fg_reads / max(fg_launches, 1))
+                                              basis_reads=fg_reads / max(fg_launches, 1), df=df)
     per_step = sweeps + solver / args.steps
     t = ms_timed / args.steps / 1e3
     return {"bound": "hbm", "achieved": round(per_step / t / 1e9, 1), "peak": pk, "peak_source": src,

@@ -48,6 +48,14 @@ def test_algorithmic_bytes(bench):
     assert d - m == nnz * 16
 
 
+def test_double_float_pass_reads_z_in_fp32(bench):
+    f = _Fake()
+    a, b = (bench.algorithmic_bytes(f, "fg_arnoldi_spmv", "mixed", basis_reads=10, df=d) for d in (False, True))
+    assert a - b == 3000.0 * 4
+    a, b = (bench.algorithmic_bytes(f, "fg_project", "mixed", basis_reads=10, df=d) for d in (False, True))
+    assert a == b
+
+
 def test_fp64_work(bench):
     f = _Fake()
     n, nnz = 3000.0, 60000.0
