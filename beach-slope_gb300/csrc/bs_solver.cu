@@ -726,7 +726,10 @@ __device__ __forceinline__ bool fg_group_sum(const Dev& D, int s, int nact, int 
 // Both levels: the last group of the scene sums the groups into tot[]; true in
 // that block.  one_level: a small scene's last block sums its blocks' values
 // itself (the order of the sums differs, so only where the solve does not
-// multiply such a difference: without the FP32 preconditioner).
+// multiply such a difference: without the FP32 preconditioner).  A column of an
+// unpreconditioned solve with one level and with two, us: 3 blocks 46.6 and 49.5,
+// 39 blocks 51.4 and 53.6, 54 blocks 52.8 and 53.0, 64 blocks 54.3 and 53.5, 79
+// blocks 58.6 and 56.9, 235 blocks 110 and 93: they cross between 54 and 64.
 #define BS_FG_ONE_LEVEL 64
 __device__ __forceinline__ bool fg_scene_sum(const Dev& D, int s, int nact, int nv, const double* vals, double* tot,
                                              bool one_level) {
@@ -1043,7 +1046,7 @@ __device__ __forceinline__ void fg_arn1_finish(const Dev& D, int s, int j, const
 // Column j, pass 1, FP64 basis: w = A z_j (z_j = the V-cycle output in sp2, kept
 // as Z_j; or v_j) into sv; one read of v_0..v_j gives h = V^T w and the Gram
 // column c = V^T v_j.
-__global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond, int* nconv) {
+__global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond) {
     BS_PDL_ENTRY();
     const int s = D.blk_scene[blockIdx.x];
     if (!fg_running(D, s)) return;
@@ -1117,12 +1120,12 @@ __global__ void __launch_bounds__(BS_THREADS, 5) k_fg_arn1(Dev D, int precond, i
 // Column j, pass 1, double-float basis: w = A z_j for the mixed V-cycle's output
 // (zf; kept as Z_j) into sv, the dots of v_0..v_j with w and v_j, and w.w.
 // Warp w takes the vectors w, w + 8, ...: 8 rows per lane loaded first, then two
-// accumulation chains, w and v_j read from shared memory (48 registers: five
-// blocks per SM).  The dots of four vectors (8 double-float values a lane) are
+// accumulation chains, w and v_j read from shared memory (48 registers, at 36
+// bytes of spills: five blocks per SM).  The dots of four vectors (8 double-float values a lane) are
 // summed over the lanes by a transposing butterfly, w.w of the eight warps by
 // one warp likewise (9 FP64 adds instead of 40), each block's value converted
-// to FP64 once for the FP64 scene sums.  Bound by HBM: 60 us for 313 MB at
-// 0.71 M particles, 0.77 of the measured copy rate.  Measured and not kept: the
+// to FP64 once for the FP64 scene sums.  Bound by HBM: 70 us for 312 MB at
+// 0.71 M particles (cold, k_fg_fin not counted), 0.65 of the measured copy rate.  Measured and not kept: the
 // basis fetched under the SpMV by bulk copies into a ring in shared memory
 // (32 KB and 64 registers: four blocks per SM; 13.86 ms per step against 13.61,
 // 4.20 against 4.06 at 0.18 M).
@@ -1703,7 +1706,7 @@ void solve_fgmres(const Dev& D, const Launch& L, int maxit, int check_every, int
         if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.fg_df ? nullptr : D.sp2, 1);   // (pass 1 of the double-float form reads zf)
         int q2 = tbegin(L, K_FG_ARN);
         if (D.fg_df) fg_pass1_df(D, L);
-        else launch_pdl(L, k_fg_arn1, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
+        else launch_pdl(L, k_fg_arn1, L.nblk_rows, BS_THREADS, 0, D, precond);
         tend(L, q2);
         q2 = tbegin(L, K_FG_ORTH);
         if (D.fg_df) launch_pdl(L, k_fg_arn2_df, L.nblk_rows + D.nscene, BS_ARN2_THREADS, 0, D, d_nconv, mgmode);
@@ -1926,7 +1929,7 @@ void fg_column(const Dev& D, const Launch& L, int precond, int mg_prec, int mgmo
     if (precond) mg_apply(D, L, mg_prec, D.fg_V, D.fg_df ? nullptr : D.sp2, 1);   // (pass 1 of the double-float form reads zf)
     int q = tbegin(L, K_FG_ARN);
     if (D.fg_df) fg_pass1_df(D, L);
-    else launch_pdl(L, k_fg_arn1, L.nblk_rows, BS_THREADS, 0, D, precond, d_nconv);
+    else launch_pdl(L, k_fg_arn1, L.nblk_rows, BS_THREADS, 0, D, precond);
     tend(L, q);
     q = tbegin(L, K_FG_ORTH);
     if (D.fg_df) launch_pdl(L, k_fg_arn2_df, L.nblk_rows + D.nscene, BS_ARN2_THREADS, 0, D, d_nconv, mgmode);

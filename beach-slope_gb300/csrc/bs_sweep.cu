@@ -113,8 +113,8 @@ __device__ __forceinline__ bool in_range(double v, bool zero = false) {
 // of one half first 539 instead of 504 us at 1.04 M rows); BS_CAND candidates
 // are loaded at once and their tests become bit masks (no branch per candidate;
 // the next batch's loads ahead cost more instructions than the wait: 531 instead
-// of 463 us); 64 registers (four blocks of 256: 72 costs 3% at 1 M rows, 48
-// spills); scene constants are rounded to FP32 on the host.  Packed FP32 instructions
+// of 463 us); 64 registers (four blocks of 256, at 60 bytes of spills in the mixed form: 72
+// cost 3% at 1 M rows, 48 spill more); scene constants are rounded to FP32 on the host.  Packed FP32 instructions
 // for two pairs at once gave nothing (439 and 439 us).
 // Both halves at 15 k, 187 k, 712 k and 1.04 M rows (64 scenes), before and now:
 // 64 and 32, 163 and 102, 382 and 293, 510 and 437 us; FP64 at 187 k 675 and
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(BS_THREADS, sizeof(T) == 4 ? 5 : 1) k_eddy(Dev
         // from the k_quot records, the differences rounded once to FP32
         const float4 q4 = D.rec0[r];
         const CorrF cf = corr_f(D, r);
-        constexpr int B = 4;   // (48 registers, five blocks of 256: 128 us without the bound, 124 with it)
+        constexpr int B = 4;   // (48 registers at 36 bytes of spills, five blocks of 256: 128 us without the bound, 124 with it)
         for (int k0 = 0; k0 < n; k0 += B) {
             int js[B];
             float z1s[B], z2s[B], Vs[B];
