@@ -409,7 +409,7 @@ void mg_tables(bs_ctx* c) {
         }
     }
     mg_sub_choose(c);
-    mg_tail_choose(c);
+    if (c->made) mg_tail_choose(c);   // (bs_create: at its end)
 }
 
 // per-scene constants that do not depend on the layout
@@ -858,6 +858,7 @@ int bs_create(int32_t nscenes, const bs_params* params, const int32_t* capacity,
             return r2;
         }
     }
+    mg_tail_choose(ctx);   // its constants last: they may do without room, the rest may not
     cudaStreamSynchronize(nullptr);   // the arrays' clearing
     ctx->made = true;
     cudaError_t e = cudaGetLastError();

@@ -24,3 +24,28 @@ def test_no_room_for_the_chip_image(monkeypatch, tmp_path):
     c.set_option("mg_tail", 1)   # room again
     assert c.get_option("mg_tail_level") == 1
     c.close()
+
+
+def test_the_image_takes_no_room_that_the_context_needs(monkeypatch, tmp_path):
+    """With just the memory that a context needs without the constants, and with
+    anything up to what it takes with them, it is made."""
+    from beachslope_gb300 import scene
+    gpu = FakeGpu(monkeypatch, tmp_path)
+    p, st, gr = scene.beach_scene(dx=0.0133)
+
+    def made(room):
+        gpu.lib.fake_room(room)
+        c = gpu.api.Context([p], [st], [gr])
+        n = C.c_size_t()
+        assert gpu.lib.bs_context_bytes(c.h, C.byref(n)) == 0
+        level = c.get_option("mg_tail_level")
+        c.close()
+        return n.value, level
+
+    total, level = made(1 << 30)
+    assert level == 1
+    bare, level = made(total * 59 // 60)
+    assert level == 0 and bare < total
+    for room in (bare, bare + 1, (bare + total) // 2, total - 1):
+        assert made(room) == (bare, 0)
+    assert made(total) == (total, 1)
