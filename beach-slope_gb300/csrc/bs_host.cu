@@ -135,6 +135,13 @@ int fail(bs_ctx* c, int code, const std::string& m) {
         if (e_ != cudaSuccess) return fail(ctx, BS_E_CUDA, std::string(#call ": ") + cudaGetErrorString(e_)); \
     } while (0)
 
+// The context's stream does not wait for the null stream by itself: nothing that
+// follows on it runs before the null stream's memsets so far.
+void order_clears(bs_ctx* ctx) {
+    cudaEventRecord(ctx->evsync, nullptr);
+    cudaStreamWaitEvent(ctx->stream, ctx->evsync, 0);
+}
+
 template <class T>
 int dalloc(bs_ctx* ctx, T** p, size_t n) {
     void* q = nullptr;
@@ -145,8 +152,7 @@ int dalloc(bs_ctx* ctx, T** p, size_t n) {
         return fail(ctx, BS_E_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
     cudaMemset(q, 0, n * sizeof(T));
-    // the context's streams do not wait for the null stream (bs_create waits once, at its end)
-    if (ctx->made) cudaStreamSynchronize(nullptr);
+    if (ctx->made) order_clears(ctx);   // (bs_create: once, at its end)
     ctx->allocs.push_back(q);
     ctx->alloc_bytes.push_back(n * sizeof(T));
     *p = (T*)q;
@@ -859,7 +865,7 @@ int bs_create(int32_t nscenes, const bs_params* params, const int32_t* capacity,
         }
     }
     mg_tail_choose(ctx);   // its constants last: they may do without room, the rest may not
-    cudaStreamSynchronize(nullptr);   // the arrays' clearing
+    order_clears(ctx);
     ctx->made = true;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

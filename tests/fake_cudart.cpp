@@ -27,6 +27,7 @@ size_t used = 0, room = (size_t)1 << 40;  // bytes of device memory
 cudaError_t last = cudaSuccess, refuse_coop = cudaSuccess;
 int sms = 152;
 bool clearing = false;   // a memset on the null stream that nothing has waited for
+bool marked = false;     // ... with an event behind it
 int early = 0;           // launches while it may still run
 std::vector<cudaLaunchConfig_t> configs;
 
@@ -173,6 +174,7 @@ cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size
 }
 cudaError_t cudaMemset(void* d, int v, size_t n) {
     clearing = true;
+    marked = false;
     return std::memset(d, v, n), cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return std::memset(d, v, n), cudaSuccess; }
@@ -185,11 +187,17 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s) {
     if (!s) clearing = false;   // (the library's own streams do not wait for the null stream)
     return cudaSuccess;
 }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) {
+    if (marked) clearing = false;
+    return cudaSuccess;
+}
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return *e = (cudaEvent_t)&token, cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t s) {
+    marked |= !s;
+    return cudaSuccess;
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.0f, cudaSuccess; }
