@@ -313,7 +313,7 @@ void mg_tail_choose(bs_ctx* c) {
     c->mgtail_level = 0;
     c->mgchip_cs = 1;
     c->mgchip_smem = 0;
-    if (!c->mgtail_on || M.exact || c->mgsub_level || c->mglev.empty()) return;
+    if (!c->mgtail_on || M.exact || c->mgsub_level || c->mglev.empty() || !c->prm[0].ppe_precond) return;
     const int prec = mg_prec_of(c);
     for (int l = 1; l <= M.nlev; ++l) {
         if (!(c->mgneed[l] & 1)) break;
@@ -343,8 +343,10 @@ void mg_tail_choose(bs_ctx* c) {
         const size_t need = (size_t)c->nscene * best * best_smem;
         if (need > c->chip_img_bytes) {
             char* img = (char*)c->D.mg.chip_img;
-            cudaStreamSynchronize(c->stream);
-            dfree(c, img);
+            if (img) {
+                cudaStreamSynchronize(c->stream);
+                dfree(c, img);
+            }
             c->D.mg.chip_img = nullptr;
             c->chip_img_bytes = 0;
             if (dalloc(c, &img, need)) return;   // no room: the separate launches

@@ -49,3 +49,20 @@ def test_the_image_takes_no_room_that_the_context_needs(monkeypatch, tmp_path):
     for room in (bare, bare + 1, (bare + total) // 2, total - 1):
         assert made(room) == (bare, 0)
     assert made(total) == (total, 1)
+
+
+def test_no_constants_without_the_preconditioner(monkeypatch, tmp_path):
+    """Solves that run no multigrid cycle (the reference's settings, the CSR
+    calls) do not allocate its constants; switching it on does."""
+    from beachslope_gb300 import scene
+    gpu = FakeGpu(monkeypatch, tmp_path)
+    p, st, gr = scene.beach_scene(dx=0.0133)
+    p.ppe_precond = 0
+    c = gpu.api.Context([p], [st], [gr])
+    n = [C.c_size_t(), C.c_size_t()]
+    assert gpu.lib.bs_context_bytes(c.h, C.byref(n[0])) == 0
+    assert c.get_option("mg_tail_level") == 0
+    c.set_option("ppe_precond", 1)
+    assert gpu.lib.bs_context_bytes(c.h, C.byref(n[1])) == 0
+    assert c.get_option("mg_tail_level") == 1 and n[1].value > n[0].value
+    c.close()
